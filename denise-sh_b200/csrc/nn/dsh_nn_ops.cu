@@ -422,33 +422,47 @@ __global__ void colsum_k(const float *dy, long long P, int N, float *part)
     }
 }
 
-/* The same with N a divisor of 1024 and a multiple of 4 (every layer): thread
- * t owns four columns (t % (N/4)) and every (1024/N)-th row of the block's
- * chunk, so a warp reads contiguous 512 bytes and 8 loads are in flight per
- * thread; the partials are combined in a fixed order.  With one thread per
- * column 32 of 256 threads work when N = 32: 2.45 ms in the 17 launches of a
- * training step on two 400 x 1200 maps, 0.52 ms with this one. */
-__global__ void __launch_bounds__(256) colsum_v4(const float4 *dy, long long P, int N, float *part)
+/* The same sums in the same order (one thread per column, rows in sequence),
+ * fed through shared memory: the whole block copies tiles of 4096 floats
+ * ahead with cp.async while the first N threads add the current one.  N a
+ * multiple of 4, at most 256.  With each column's thread loading its own rows
+ * 32 of 256 threads worked when N = 32: 2.45 ms in the 17 launches of a
+ * training step on two 400 x 1200 maps; now bound by the chain of additions. */
+constexpr int CS_TILE = 4096;
+__global__ void __launch_bounds__(256) colsum_tiles(const float *dy, long long P, int N, float *part)
 {
-    __shared__ float4 sh[256];
-    const int nv = N / 4, lanes = 256 / nv, c = threadIdx.x % nv, lane = threadIdx.x / nv;
+    __shared__ __align__(16) float sh[2][CS_TILE];
     const long long rows = (P + gridDim.x - 1) / gridDim.x;
     const long long r0 = (long long)blockIdx.x * rows, r1 = min(P, r0 + rows);
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (long long p = r0 + lane; p < r1; p += lanes) {
-        const float4 v = __ldg(dy + p * nv + c);
-        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-    }
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    if (lane == 0) {
-        for (int k = 1; k < lanes; k++) {
-            const float4 v = sh[k * nv + c];
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    const int tr = CS_TILE / N;                          /* rows of a tile */
+    const long long ntile = r1 > r0 ? (r1 - r0 + tr - 1) / tr : 0;
+    auto fetch = [&](long long t) {
+        if (t < ntile) {
+            const long long p = r0 + t * tr;
+            const int n4 = (int)(min((long long)tr, r1 - p) * N / 4);
+            const float4 *src = reinterpret_cast<const float4 *>(dy + p * N);
+            for (int k = threadIdx.x; k < n4; k += blockDim.x) {
+                const uint32_t d = (uint32_t)__cvta_generic_to_shared(&sh[t & 1][4 * k]);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + k) : "memory");
+            }
         }
-        reinterpret_cast<float4 *>(part + (long long)blockIdx.x * N)[c] = s;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float s = 0.0f;
+    fetch(0);
+    for (long long t = 0; t < ntile; t++) {
+        fetch(t + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const int n = (int)min((long long)tr, r1 - (r0 + t * tr));
+        if ((int)threadIdx.x < N) {
+            const float *col = &sh[t & 1][threadIdx.x];
+#pragma unroll 16
+            for (int p = 0; p < n; p++) s += col[p * N];
+        }
+        __syncthreads();
     }
+    if ((int)threadIdx.x < N) part[(long long)blockIdx.x * N + threadIdx.x] = s;
 }
 
 /* g[n] += sum over blocks of part[b*stride + n], blocks in order */
@@ -456,6 +470,7 @@ __global__ void sum_parts_k(const float *part, int nblocks, int N, int stride, f
 {
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
         float s = 0.0f;
+#pragma unroll 16
         for (int b = 0; b < nblocks; b++) s += part[(long long)b * stride + n];
         g[n] += s;
     }
@@ -674,8 +689,8 @@ extern "C" int dsh_nn_head_bwd(const float *dout, const void *x, long long P, in
 extern "C" int dsh_nn_colsum(const float *dy, long long P, int N, float *g, float *part, void *stream)
 {
     if (!dy || !g || !part || P <= 0 || N <= 0) return DSH_NN_ERR_PARAM;
-    if (N % 4 == 0 && N <= 1024 && 1024 % N == 0 && al16(dy) && al16(part))
-        colsum_v4<<<RED_BLOCKS, 256, 0, ST>>>((const float4 *)dy, P, N, part);
+    if (N % 4 == 0 && N <= 256 && al16(dy))
+        colsum_tiles<<<RED_BLOCKS, 256, 0, ST>>>(dy, P, N, part);
     else
         colsum_k<<<RED_BLOCKS, 256, 0, ST>>>(dy, P, N, part);
     sum_parts_k<<<(N + 255) / 256, 256, 0, ST>>>(part, RED_BLOCKS, N, N, g);
