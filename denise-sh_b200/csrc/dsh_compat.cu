@@ -245,6 +245,7 @@ StepArgs base_args(const float *hc)
     for (int k = 0; k <= 6; k++) a.hc[k] = hc[k];
     a.dt = DT; a.dh = DH;
     a.inv_dh = (float)(1.0 / (double)DH);
+    a.rdh_d = 1.0 / (double)DH;
     a.dhi_el = DT / DH;
     a.dhi_visc = (float)(1.0 / (double)DH);
     a.dthalbe = (float)((double)DT / 2.0);

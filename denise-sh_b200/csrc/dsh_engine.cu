@@ -362,6 +362,13 @@ __global__ void gather_dense_kernel(int nx, int ny, int pitch, const float *src,
 
 __global__ void set_int_kernel(int *p, int v) { *p = v; }
 
+/* div_dh's product form against the division for every significand of x (2^23 threads) */
+__global__ void rdh_check(float dh, float zh, float zl, int *differ)
+{
+    const float x = __uint_as_float(0x3f800000u | (blockIdx.x * blockDim.x + threadIdx.x));
+    if (rdh_product(x, zh, zl) != x / dh) atomicOr(differ, 1);
+}
+
 }  // namespace
 
 /* ======================= context (struct dsh_ctx: dsh_engine_int.h) ======================= */
@@ -541,6 +548,18 @@ extern "C" dsh_ctx *dsh_create(const dsh_params *p, int device, int *status)
     if (cudaMalloc(&ctx->d_l2, (size_t)ctx->S * sizeof(double)) != cudaSuccess) return bail(DSH_ERR_OOM);
     if (cudaMalloc(&ctx->d_wemax, (size_t)ctx->S * sizeof(unsigned)) != cudaSuccess) return bail(DSH_ERR_OOM);
     if (cudaMalloc(&ctx->d_offs, 4 * (size_t)ctx->S * sizeof(long long)) != cudaSuccess) return bail(DSH_ERR_OOM);
+    if (!dh_pow2(p->dh) && p->dh >= 0x1p-20f && p->dh <= 0x1p20f) {
+        ctx->rdh_h = (float)(1.0 / (double)p->dh);
+        ctx->rdh_l = (float)(1.0 / (double)p->dh - (double)ctx->rdh_h);
+        ctx->rdh_lo = std::max(std::max(0x1p-100f, 0x1p-100f * p->dh), 0x1p-124f / std::fabs(ctx->rdh_l));
+        ctx->rdh_hi = std::min(0x1p100f, 0x1p100f * p->dh);
+        int differ = 1;
+        rdh_check<<<(1 << 23) / 256, 256>>>(p->dh, ctx->rdh_h, ctx->rdh_l, ctx->d_status);
+        if (cudaMemcpy(&differ, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+            cudaMemset(ctx->d_status, 0, sizeof(int)) != cudaSuccess)
+            return bail(DSH_ERR_CUDA);
+        ctx->rdh_on = !differ && ctx->rdh_lo < ctx->rdh_hi;
+    }
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(DSH_ERR_CUDA);
     memset(&ctx->stats, 0, sizeof(ctx->stats));
     if (status) *status = DSH_OK;
@@ -718,6 +737,9 @@ extern "C" int dsh_set_model(dsh_ctx *ctx, const float *vs, const float *rho, co
     const size_t vlen = 2 * DSH_MAX_FW + 1;
     std::vector<float> pmlh(12 * vlen);
     for (int k = 0; k < 12; k++) memcpy(&pmlh[k * vlen], vecs[k], vlen * sizeof(float));
+    ctx->pml_k1 = 1;
+    for (int k = 0; k < 12; k += 3)
+        for (int i = 1; i <= 2 * p.fw; i++) ctx->pml_k1 &= vecs[k][i] == 1.0f;
     CK(cudaMemcpyAsync(ctx->pml, pmlh.data(), pmlh.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->st));
     /* the model in, the coefficient fields formed on the device */
     int rc;
@@ -899,20 +921,22 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
         }
     }
 
-    /* one int buffer: fixed tables, then 8 variable sections of capacity cp */
+    /* one int buffer: fixed tables, then 9 variable sections of capacity cp */
+    std::vector<int> gsid(grp_pt.size());            /* the source of a group with one member, else -1 */
+    for (size_t g = 0; g < gsid.size(); g++) gsid[g] = grp_beg[g + 1] == grp_beg[g] + 1 ? src_id[grp_beg[g]] : -1;
     const long long F = 3LL * (S + 1) + 3LL * S * (T + 1) + 2LL * S * (FT + 1);
     const long long maxlen = (long long)std::max({grp_pt.size(), grp_beg.size(), src_id.size(), rec_pt.size(),
                                                   gpk.size(), rpk.size(), rid.size(), fvids.size()}) + 1;
     bool realloc = false;
-    if (F + 8 * maxlen > ctx->geo_cap) {
+    if (F + 9 * maxlen > ctx->geo_cap) {
         cudaFree(ctx->d_geo);
         ctx->d_geo = nullptr;
-        const long long cp_old = ctx->geo_cap > F ? (ctx->geo_cap - F) / 8 : 0;
-        ctx->geo_cap = F + 8 * std::max(maxlen, 2 * cp_old);
+        const long long cp_old = ctx->geo_cap > F ? (ctx->geo_cap - F) / 9 : 0;
+        ctx->geo_cap = F + 9 * std::max(maxlen, 2 * cp_old);
         CK(cudaMalloc(&ctx->d_geo, (size_t)ctx->geo_cap * sizeof(int)));
         realloc = true;
     }
-    const long long cp = (ctx->geo_cap - F) / 8;
+    const long long cp = (ctx->geo_cap - F) / 9;
     int *G = ctx->d_geo;
     ctx->d_fgrp_off = G; ctx->d_agrp_off = G + (S + 1); ctx->d_rec_off = G + 2 * (S + 1);
     ctx->d_ftile = G + 3 * (S + 1); ctx->d_atile = ctx->d_ftile + S * (T + 1); ctx->d_rtile = ctx->d_atile + S * (T + 1);
@@ -921,6 +945,7 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
     ctx->d_rid = ctx->d_rpk + cp;
     ctx->d_fvoff = ctx->d_rtile + S * (T + 1); ctx->d_avoff = ctx->d_fvoff + S * (FT + 1);
     ctx->d_fvids = ctx->d_rid + cp;
+    ctx->d_gsid = ctx->d_fvids + cp;
     ctx->fvg_ntiles = FT;
     ctx->ntiles = T;
     ctx->fused_inject = fused && getenv("DSH_NO_FUSED_INJECT") == nullptr;
@@ -930,7 +955,7 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
     put(3 * (S + 1), ftile); put(3 * (S + 1) + S * (T + 1), atile); put(3 * (S + 1) + 2 * S * (T + 1), rtile);
     put(F, grp_pt); put(F + cp, grp_beg); put(F + 2 * cp, src_id); put(F + 3 * cp, rec_pt);
     put(F + 4 * cp, gpk); put(F + 5 * cp, rpk); put(F + 6 * cp, rid);
-    put(3 * (S + 1) + 3 * S * (T + 1), fvoff); put(F + 7 * cp, fvids);
+    put(3 * (S + 1) + 3 * S * (T + 1), fvoff); put(F + 7 * cp, fvids); put(F + 8 * cp, gsid);
     CK(cudaMemcpyAsync(ctx->d_geo, host.data(), (size_t)ctx->geo_cap * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
     WAIT(ctx);
 
@@ -1034,6 +1059,9 @@ StepArgs step_args(dsh_ctx *ctx, Pass pass)
     for (int k = 0; k < 7; k++) a.hc[k] = ctx->hc[k];
     a.dt = p.dt; a.dh = p.dh;
     a.inv_dh = (float)(1.0 / (double)p.dh);
+    a.pml_k1 = ctx->pml_k1;
+    a.rdh_on = ctx->rdh_on; a.rdh_h = ctx->rdh_h; a.rdh_l = ctx->rdh_l; a.rdh_lo = ctx->rdh_lo; a.rdh_hi = ctx->rdh_hi;
+    a.rdh_d = 1.0 / (double)p.dh;
     a.dhi_el = p.dt / p.dh;
     a.dhi_visc = (float)(1.0 / (double)p.dh);
     a.dthalbe = (float)((double)p.dt / 2.0);
@@ -1080,6 +1108,7 @@ StepArgs step_args(dsh_ctx *ctx, Pass pass)
     a.tl.ntiles = ctx->ntiles;
     a.tl.ntx = (p.nx + 4 * BX - 1) / (4 * BX);
     a.tl.gpt = ctx->d_gpk; a.tl.gbeg = ctx->d_grp_beg; a.tl.src_id = ctx->d_src_id;
+    a.tl.gsid = ctx->d_gsid; a.tl.rec_pt = ctx->d_rec_pt;
     a.tl.roff = ctx->d_rtile; a.tl.rpt = ctx->d_rpk; a.tl.rid = ctx->d_rid; a.tl.rec_off = ctx->d_rec_off;
     a.tl.seis = ctx->d_seis; a.tl.seis_off = ctx->d_offs + ctx->S;
     if (pass == P_ADJ) {
@@ -1293,6 +1322,11 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
     const int sr = s_rows();
     dim3 block(BX, sr, 1);
     dim3 grid((unsigned)((p.nx + 4 * BX - 1) / (4 * BX)), (unsigned)((p.ny + sr - 1) / sr), (unsigned)nb);
+    if (sa.tl.on && sa.tl.sample) {          /* the stress launch samples the receivers (sample_block) */
+        sa.tl.samp_by = (int)grid.y;
+        sa.tl.sample = 0;
+        grid.y += 1;
+    }
     dim3 vgrid, vblock;
     v_shape(ctx, vp, nb, &vgrid, &vblock);
     /* velocity and stress kernels overlap their prologues with the

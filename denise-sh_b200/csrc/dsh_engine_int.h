@@ -45,6 +45,9 @@ struct dsh_ctx {
     float *pml = nullptr;
     float *sums = nullptr;                /* sum_u, sum_rho, out_a, out_b (dense pitched) */
     float hc[7] = {0}, bip[4] = {0}, bjm[4] = {0}, cip[4] = {0}, cjm[4] = {0}, cnorm[2] = {0};
+    int pml_k1 = 0;                       /* every CPML stretching K is 1 */
+    int rdh_on = 0;                       /* div_dh's product form gives RN(x / DH) (see dsh_kernels.cuh) */
+    float rdh_h = 0.0f, rdh_l = 0.0f, rdh_lo = 0.0f, rdh_hi = 0.0f;
     int model_set = 0;
     float *fwd = nullptr;
     long long fwd_slot_stride = 0, fwd_step_stride = 0;
@@ -61,6 +64,7 @@ struct dsh_ctx {
     int *d_ftile, *d_atile, *d_rtile, *d_gpk, *d_rpk, *d_rid;
     int ntiles = 0, fused_inject = 0;
     int *d_fvoff = nullptr, *d_avoff = nullptr, *d_fvids = nullptr;   /* fused-tile injection lists */
+    int *d_gsid = nullptr;                /* per source group: its source if it has one, else -1 */
     int fvg_ntiles = 0;
     long long *d_offs = nullptr;          /* sig_off[S], seis_off[S], obs_off[S], out_off[S] */
     float *d_sig = nullptr, *d_seis = nullptr, *d_res = nullptr, *d_obs = nullptr, *d_tmp = nullptr;

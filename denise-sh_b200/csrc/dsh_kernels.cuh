@@ -65,17 +65,20 @@ struct TileLists {
     const int *gpt;              /* packed point (j << 16 | i) of group g */
     const int *gbeg;             /* members of group g: src_id[gbeg[g] .. gbeg[g+1]) */
     const int *src_id;
+    const int *gsid;             /* the source of group g where it has one member, else -1 */
     const float *sig;            /* signal of source sid at step nt: sig[sig_off[s] + sid*sig_ss + (nt-1)*sig_ts] */
     const long long *sig_off;
     long long sig_ss, sig_ts;
     const int *roff;             /* [slot][ntiles+1] -> receiver entries of a tile */
     const int *rpt;              /* packed point of receiver entry e */
+    const int *rec_pt;           /* field offsets of the receivers in their own order (from rec_off[slot]) */
     const int *rid;              /* receiver index (within its slot) of entry e */
     const int *rec_off;          /* [slot+1]: receivers of slot s are rec_off[s] .. rec_off[s+1] */
     float *seis;                 /* slot s: seis[seis_off[s] + (nt-1)*ntr_s + r] */
     const long long *seis_off;
     int ntiles;
     int ntx;                     /* list tiles along x: ceil(nx / 128); tile of (i, j) = ((j-1)/8)*ntx + (i-1)/128 */
+    int samp_by;                 /* kernel pair: block row of the stress launch that samples the receivers, 0: none */
     int on;                      /* fused path active (all positions inside the grid) */
     int sample;
 };
@@ -96,6 +99,9 @@ struct StepArgs {
     long long slot_stride;       /* floats between consecutive shot slots */
     float hc[7];
     float dt, dh, inv_dh, dhi_el, dhi_visc, dthalbe;
+    int rdh_on, pml_k1;          /* div_dh's product form proven for this DH; every CPML K is 1 */
+    float rdh_h, rdh_l, rdh_lo, rdh_hi;
+    double rdh_d;                /* 1 / DH */
     PmlCoef pml;
     /* per-slot state (slot 0 base; slot s at + s*slot_stride) */
     float *vy, *sxy, *syz, *r, *q, *psi_vxx, *psi_vyy_v, *psi_sxx, *psi_syy;
@@ -283,10 +289,160 @@ __device__ __forceinline__ void set_lane(float4 &v, int k, float x)
  * every step (mod = NT > s), the case of full storage */
 __device__ __forceinline__ long long store_idx(int s, int mod) { return s < mod ? s : s % mod; }
 
+/* Keeps the compiler from computing the divisions of a branch ahead of it and
+ * selecting (it takes them for cheap; with values ahead of the wavefront,
+ * which are denormal, each takes the division's slow path). */
+__device__ __forceinline__ void stay_in_branch() { asm volatile("" ::: "memory"); }
+
 /* x / DH: when DH is a power of two the product with the exact reciprocal is
- * the same correctly rounded value, so P2 kernels multiply. */
+ * the same correctly rounded value, so P2 kernels multiply.  Otherwise, when
+ * the host set rdh_on, the division by a divisor known in advance of
+ * Brisebarre, Muller and Raina (IEEE Trans. Comput. 53(8), 2004):
+ *   q = RN(x zh + RN(x zl)),  zh = RN(1/DH), zl = RN(1/DH - zh),
+ * a product and a fused multiply-add.  Whether it gives RN(x/DH) depends only
+ * on x's significand as long as nothing under- or overflows, so dsh_create
+ * compares it with the division for all 2^23 significands (rdh_check) and
+ * rdh_lo <= |x| <= rdh_hi keeps RN(x zl) and q in the normal range; zeros
+ * keep their sign.  Everything else (the tiny values ahead of a wavefront
+ * above all) takes div_dh_double.  Per step of a 2000 x 800 grid, FDORDER 8,
+ * DH 0.6 the divisions cost 5.5 us, these 0.6. */
+/* RN(x/DH) through a quotient in double precision, corrected once (Markstein,
+ * IBM J. Res. Dev. 34(1), 1990).  Its relative error is at most 2^-52, while a
+ * quotient of two floats that is no midpoint of two floats is at least 2^-49
+ * away from one, and a quotient that is a midpoint (only possible for a
+ * denormal result) has at most 25 bits, is a double and comes out exactly:
+ * so rounding it to float gives the correctly rounded quotient. */
+__device__ __forceinline__ float div_dh_double(float x, const StepArgs &a)
+{
+    const double xd = (double)x, dh = (double)a.dh, q = xd * a.rdh_d;
+    return isfinite(x) ? (float)__fma_rn(__fma_rn(-q, dh, xd), a.rdh_d, q) : x;
+}
+
+__device__ __forceinline__ float rdh_product(float x, float zh, float zl) { return __fmaf_rn(x, zh, __fmul_rn(x, zl)); }
+
 template <bool P2>
-__device__ __forceinline__ float div_dh(float x, const StepArgs &a) { return P2 ? x * a.inv_dh : x / a.dh; }
+__device__ __forceinline__ float div_dh(float x, const StepArgs &a)
+{
+    if (P2) return x * a.inv_dh;
+    const float ax = fabsf(x);
+    if (a.rdh_on && ((ax >= a.rdh_lo && ax <= a.rdh_hi) || ax == 0.0f))
+        return ax == 0.0f ? x : rdh_product(x, a.rdh_h, a.rdh_l);
+    stay_in_branch();
+    return div_dh_double(x, a);
+}
+
+/* four quotients with one test */
+template <bool P2>
+__device__ __forceinline__ void div4_dh(float *x, const StepArgs &a)
+{
+    if (P2) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[k] = x[k] * a.inv_dh;
+        return;
+    }
+    bool in = a.rdh_on != 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float ax = fabsf(x[k]);
+        in = in && ((ax >= a.rdh_lo && ax <= a.rdh_hi) || ax == 0.0f);
+    }
+    if (in) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[k] = x[k] == 0.0f ? x[k] : rdh_product(x[k], a.rdh_h, a.rdh_l);
+    } else {
+        stay_in_branch();
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[k] = div_dh_double(x[k], a);
+    }
+}
+
+/* CPML recursion psi = b psi + a d, d = d/K + psi (update_v_PML.c:51-198) of
+ * points k0 <= k < k1 of a thread's four in an x strip: coefficients and psi
+ * at consecutive addresses.  All loads are issued before the first use. */
+__device__ __forceinline__ void cpml_x4(float *d, float *p, const float *K, const float *ca, const float *cb, int k0, int k1,
+                                        bool k_one)
+{
+    float ps[4], a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (k >= k0 && k < k1) { ps[k] = p[k]; a[k] = __ldg(ca + k); b[k] = __ldg(cb + k); }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (k >= k0 && k < k1) { ps[k] = b[k] * ps[k] + a[k] * d[k]; p[k] = ps[k]; }
+    if (!k_one) {
+        stay_in_branch();
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (k >= k0 && k < k1) d[k] = d[k] / __ldg(K + k);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (k >= k0 && k < k1) d[k] = d[k] + ps[k];
+}
+/* the same of the thread's points in a depth strip: one coefficient triple, psi a float4 */
+__device__ __forceinline__ void cpml_y4(float *d, float *p, float4 ps, float K, float ca, float cb, int nvalid, bool k_one)
+{
+    float4 t;
+    t.x = cb * ps.x + ca * d[0]; t.y = cb * ps.y + ca * d[1];
+    t.z = cb * ps.z + ca * d[2]; t.w = cb * ps.w + ca * d[3];
+    st4m(p, t, nvalid);
+    if (!k_one) {
+        stay_in_branch();
+#pragma unroll
+        for (int k = 0; k < 4; k++) d[k] = d[k] / K;
+    }
+    d[0] = d[0] + t.x; d[1] = d[1] + t.y; d[2] = d[2] + t.z; d[3] = d[3] + t.w;
+}
+
+/* coefficient vectors (index 1..2fw) of one axis of a kernel */
+struct CpmlAxis {
+    const float *K, *a, *b;
+};
+
+/* The CPML strips of a thread's four points: dx the x derivatives, dy the
+ * depth derivatives, px the x-strip memory of row j, py the depth-strip
+ * memory (slot base), yt / yb the coefficients of the top and bottom strip.
+ * The depth strip's loads are issued before the x strip is computed, so a
+ * corner pays one memory latency; when each point loaded, updated and stored
+ * its own value in turn, the stores kept the next loads back and a thread paid
+ * up to eight latencies in a row: 160 x 80, FDORDER 4: 11.1 us per step, 6.2
+ * without strips; 2000 x 800, FDORDER 8, L 3: 31.3 and 23.7. */
+__device__ __forceinline__ void cpml4(const StepArgs &s, int i0, int j, int nvalid, float *dx, float *dy, float *px, float *py,
+                                      const CpmlAxis &x, const CpmlAxis &yt, const CpmlAxis &yb)
+{
+    const int fw = s.fw, nx = s.nx, ny = s.ny;
+    const bool k_one = s.pml_k1 != 0;
+    const bool left = i0 <= fw, right = i0 + 3 >= nx - fw + 1;
+    const bool top = !s.free_surf && j <= fw, bottom = j >= ny - fw + 1;
+    const int hr = i0 - nx + 2 * fw;                     /* right strip: coefficient index of point k = 0 */
+    float4 ps = make_float4(0.f, 0.f, 0.f, 0.f);
+    float K = 1.f, ca = 0.f, cb = 0.f;
+    float *pr = py;
+    if (top || bottom) {
+        const int h = top ? j : j - ny + 2 * fw;
+        const CpmlAxis &y = top ? yt : yb;
+        pr = py + (long long)(h - 1) * s.pitch + (i0 - 1 + HX);
+        ps = ld4(pr);
+        ca = __ldg(y.a + h);
+        cb = __ldg(y.b + h);
+        if (!k_one) K = __ldg(y.K + h);
+    }
+    if (left || right) {
+        const int h = left ? i0 : hr;
+        cpml_x4(dx, px + (h - 1), x.K + h, x.a + h, x.b + h, left ? 0 : max(0, nx - fw + 1 - i0),
+                left ? min(nvalid, fw - i0 + 1) : nvalid, k_one);
+        if (left && right)                               /* NX < 2 FW + 3 */
+            cpml_x4(dx, px + (hr - 1), x.K + hr, x.a + hr, x.b + hr, max(0, nx - fw + 1 - i0), nvalid, k_one);
+    }
+    if (top || bottom) {
+        cpml_y4(dy, pr, ps, K, ca, cb, nvalid, k_one);
+        if (top && bottom) {                             /* NY < 2 FW */
+            const int h = j - ny + 2 * fw;
+            pr = py + (long long)(h - 1) * s.pitch + (i0 - 1 + HX);
+            cpml_y4(dy, pr, ld4(pr), k_one ? 1.f : __ldg(yb.K + h), __ldg(yb.a + h), __ldg(yb.b + h), nvalid, k_one);
+        }
+    }
+}
 
 /*
  * Velocity half-step (update_v_PML.c:51-198 for FDORDER = FDO): per point
@@ -340,7 +496,69 @@ struct SharedTaps {
     }
 };
 
-template <int FDO, int FLAGS, bool P2, class Taps = GlobalTaps<>, bool CG = false>
+/* What the lists of a tile hold for a thread's four points, found before the
+ * previous kernel's results are waited for (the lists and signals do not
+ * depend on them): at most one source point with one source (its signal at
+ * this step in sig, the point in inj), at most one receiver (the address of
+ * its sample, the point in the two low bits).  A thread with more walks the
+ * lists after the update (INJ_MANY, REC_MANY). */
+constexpr int INJ_NONE = 0, INJ_ONE = 1, INJ_MANY = 5;
+constexpr unsigned long long REC_MANY = 1;           /* no address: sample addresses are 4-byte aligned and > 4 */
+struct PointWork {
+    int inj;
+    float sig;
+    unsigned long long rec;
+};
+
+/* The lanes of a warp (one row j, four points each) read 32 list entries at a
+ * time and pass on those of their row.  Each thread walking its tile's lists
+ * by itself after the update cost a chain of five dependent loads per step in
+ * the tiles that hold a source or a receiver: 160 x 80, FDORDER 4, one
+ * source and 32 receivers: 1.3 us of 11.1 us per step. */
+template <bool SAMPLE>
+__device__ __forceinline__ void point_lists(const StepArgs &a, int nt, int i0, int j, int slot, int tg0, int tg1, int tr0,
+                                            int tr1, PointWork *w)
+{
+    w->inj = INJ_NONE;
+    w->sig = 0.0f;
+    w->rec = 0;
+    if (tg0 >= tg1 && !(SAMPLE && tr0 < tr1)) return;    /* the tile's ranges: the same in all lanes */
+    const int ln = threadIdx.x & 31;
+    const int live = min(32, (a.nx - (i0 - 4 * ln)) / 4 + 1);      /* lanes inside the grid */
+    const unsigned mask = live >= 32 ? 0xffffffffu : (1u << live) - 1;
+    for (int base = tg0; base < tg1; base += live) {
+        const int pk = base + ln < tg1 ? __ldg(a.tl.gpt + base + ln) : 0;
+        const int sl = base + ln < tg1 ? __ldg(a.tl.gsid + base + ln) : 0;
+        const float *sig = a.tl.sig + a.tl.sig_off[slot] + (long long)(min(nt, a.nt_last) - 1) * a.tl.sig_ts;
+        unsigned m = __ballot_sync(mask, (int)((unsigned)pk >> 16) == j);
+        while (m) {
+            const int l = __ffs(m) - 1;
+            m &= m - 1;
+            const int k = (__shfl_sync(mask, pk, l) & 0xffff) - i0, sid = __shfl_sync(mask, sl, l);
+            if (k < 0 || k > 3) continue;
+            if (w->inj != INJ_NONE || sid < 0) { w->inj = INJ_MANY; continue; }
+            w->inj = INJ_ONE + k;
+            w->sig = __ldg(sig + (long long)sid * a.tl.sig_ss);
+        }
+    }
+    if (!SAMPLE) return;
+    for (int base = tr0; base < tr1; base += live) {
+        const int pk = base + ln < tr1 ? __ldg(a.tl.rpt + base + ln) : 0;
+        unsigned m = __ballot_sync(mask, (int)((unsigned)pk >> 16) == j);
+        while (m) {
+            const int l = __ffs(m) - 1;
+            m &= m - 1;
+            const int k = (__shfl_sync(mask, pk, l) & 0xffff) - i0;
+            if (k < 0 || k > 3) continue;
+            if (w->rec) { w->rec = REC_MANY; continue; }
+            const int r0 = a.tl.rec_off[slot], ntr = a.tl.rec_off[slot + 1] - r0;
+            const float *sm = a.tl.seis + a.tl.seis_off[slot] + (long long)(nt - 1) * ntr + __ldg(a.tl.rid + base + l);
+            w->rec = (unsigned long long)sm | (unsigned)k;
+        }
+    }
+}
+
+template <int FDO, int FLAGS, bool P2, class Taps = GlobalTaps<>, bool CG = false, bool SAMPLE = (FLAGS & VF_ADJOINT) == 0>
 __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, int j, int slot, int tile,
                                        const Taps &taps = Taps())
 {
@@ -366,7 +584,7 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
     if (a.tl.on) {
         const int *go = a.tl.goff + (long long)slot * (a.tl.ntiles + 1) + tile;
         tg0 = __ldg(go); tg1 = __ldg(go + 1);
-        if (a.tl.sample) {
+        if (SAMPLE && a.tl.sample) {
             const int *ro = a.tl.roff + (long long)slot * (a.tl.ntiles + 1) + tile;
             tr0 = __ldg(ro); tr1 = __ldg(ro + 1);
         }
@@ -376,6 +594,8 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
         const long long k = store_idx(max(a.nt_total - nt, 0), a.fwd_mod);
         f4 = ldcs4(a.fwd + (long long)slot * a.fwd_slot_stride + k * a.fwd_step_stride + drow + col0);
     }
+    PointWork pw;
+    point_lists<SAMPLE>(a, nt, i0, j, slot, tg0, tg1, tr0, tr1, &pw);
     pdl_wait();                              /* stresses of the previous step are complete */
     pdl_trigger();
 
@@ -394,72 +614,68 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
        warp almost everywhere: one branch instead of four tests per point) */
     const bool in_pml = a.fw > 0 && (i0 <= a.fw || i0 + 3 >= a.nx - a.fw + 1 || (!a.free_surf && j <= a.fw) ||
                                      j >= a.ny - a.fw + 1);
+    float dx[4], dy[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const int i = i0 + k;
-        float sxy_x, syy_y;
 #pragma unroll
         for (int m = 1; m <= H; m++) {
             const int my = (FDO == 12 && m == 6 && a.fd12_compat) ? 5 : m;
             float tx = a.hc[m] * (xs[4 * NL + k + m - 1] - xs[4 * NL + k - m]);
             float ty = a.hc[my] * (get(ys[H + m - 1], k) - get(ys[H - m], k));
-            if (m == 1) { sxy_x = tx; syy_y = ty; }
-            else { sxy_x = sxy_x + tx; syy_y = syy_y + ty; }
+            if (m == 1) { dx[k] = tx; dy[k] = ty; }
+            else { dx[k] = dx[k] + tx; dy[k] = dy[k] + ty; }
         }
-        const int fw = a.fw;
-        if (in_pml && i <= a.nx) {
-            if (i <= fw) {
-                float *p = a.psi_vxx + so + (long long)(j - 1) * 2 * fw + (i - 1);
-                float ps = __ldg(a.pml.b_x + i) * *p + __ldg(a.pml.a_x + i) * sxy_x;
-                *p = ps;
-                sxy_x = sxy_x / __ldg(a.pml.K_x + i) + ps;
-            }
-            if (i >= a.nx - fw + 1) {
-                const int h1 = i - a.nx + 2 * fw;
-                float *p = a.psi_vxx + so + (long long)(j - 1) * 2 * fw + (h1 - 1);
-                float ps = __ldg(a.pml.b_x + h1) * *p + __ldg(a.pml.a_x + h1) * sxy_x;
-                *p = ps;
-                sxy_x = sxy_x / __ldg(a.pml.K_x + h1) + ps;
-            }
-            if (!a.free_surf && j <= fw) {
-                float *p = a.psi_vyy_v + so + (long long)(j - 1) * pitch + (col0 + k);
-                float ps = __ldg(a.pml.b_y + j) * *p + __ldg(a.pml.a_y + j) * syy_y;
-                *p = ps;
-                syy_y = syy_y / __ldg(a.pml.K_y + j) + ps;
-            }
-            if (j >= a.ny - fw + 1) {
-                const int h1 = j - a.ny + 2 * fw;
-                float *p = a.psi_vyy_v + so + (long long)(h1 - 1) * pitch + (col0 + k);
-                float ps = __ldg(a.pml.b_y + h1) * *p + __ldg(a.pml.a_y + h1) * syy_y;
-                *p = ps;
-                syy_y = syy_y / __ldg(a.pml.K_y + h1) + ps;
-            }
-        }
-        const float b = get(b4, k);
-        const float s = sxy_x + syy_y;
-        if (!(FLAGS & VF_ADJOINT)) set(acc4, k, div_dh<P2>(b * s, a));
-        set(vy4, k, get(vy4, k) + div_dh<P2>(b * a.dt * s, a));
+    }
+    if (in_pml) {
+        const CpmlAxis cx{a.pml.K_x, a.pml.a_x, a.pml.b_x}, cy{a.pml.K_y, a.pml.a_y, a.pml.b_y};
+        cpml4(a, i0, j, nvalid, dx, dy, a.psi_vxx + so + (long long)(j - 1) * 2 * a.fw, a.psi_vyy_v + so, cx, cy, cy);
+    }
+    /* the acceleration is formed where a pass uses it */
+    if (!(FLAGS & VF_ADJOINT) && ((FLAGS & (VF_HESS | VF_ACC_OUT)) || a.fwd)) {
+        float q[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) q[k] = get(b4, k) * (dx[k] + dy[k]);
+        div4_dh<P2>(q, a);
+        acc4 = make_float4(q[0], q[1], q[2], q[3]);
+    }
+    {
+        float q[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) q[k] = get(b4, k) * a.dt * (dx[k] + dy[k]);
+        div4_dh<P2>(q, a);
+#pragma unroll
+        for (int k = 0; k < 4; k++) set(vy4, k, get(vy4, k) + q[k]);
     }
 
     /* ---- fused injection (sources in order per point) and sampling ---- */
-    for (int g = tg0; g < tg1; g++) {
-        const int pk = __ldg(a.tl.gpt + g);
-        const int gi = pk & 0xffff, gj = pk >> 16;
-        if (gj == j && gi >= i0 && gi < i0 + 4) {
-            float v = lane(vy4, gi - i0);
-            const float *sg = a.tl.sig + a.tl.sig_off[slot] + (long long)(nt - 1) * a.tl.sig_ts;
-            for (int e = __ldg(a.tl.gbeg + g); e < __ldg(a.tl.gbeg + g + 1); e++)
-                v = v + sg[(long long)__ldg(a.tl.src_id + e) * a.tl.sig_ss];
-            set_lane(vy4, gi - i0, v);
+    if (pw.inj == INJ_ONE + 0) vy4.x = vy4.x + pw.sig;
+    else if (pw.inj == INJ_ONE + 1) vy4.y = vy4.y + pw.sig;
+    else if (pw.inj == INJ_ONE + 2) vy4.z = vy4.z + pw.sig;
+    else if (pw.inj == INJ_ONE + 3) vy4.w = vy4.w + pw.sig;
+    else if (pw.inj == INJ_MANY) {
+        for (int g = tg0; g < tg1; g++) {
+            const int pk = __ldg(a.tl.gpt + g);
+            const int gi = pk & 0xffff, gj = pk >> 16;
+            if (gj == j && gi >= i0 && gi < i0 + 4) {
+                float v = lane(vy4, gi - i0);
+                const float *sg = a.tl.sig + a.tl.sig_off[slot] + (long long)(nt - 1) * a.tl.sig_ts;
+                for (int e = __ldg(a.tl.gbeg + g); e < __ldg(a.tl.gbeg + g + 1); e++)
+                    v = v + sg[(long long)__ldg(a.tl.src_id + e) * a.tl.sig_ss];
+                set_lane(vy4, gi - i0, v);
+            }
         }
     }
-    if (tr1 > tr0) {
-        const int r0 = a.tl.rec_off[slot], ntr = a.tl.rec_off[slot + 1] - r0;
-        float *sm = a.tl.seis + a.tl.seis_off[slot] + (long long)(nt - 1) * ntr;
-        for (int e = tr0; e < tr1; e++) {
-            const int pk = __ldg(a.tl.rpt + e);
-            const int ri = pk & 0xffff, rj = pk >> 16;
-            if (rj == j && ri >= i0 && ri < i0 + 4) sm[__ldg(a.tl.rid + e)] = lane(vy4, ri - i0);
+    if (SAMPLE && pw.rec) {
+        if (pw.rec != REC_MANY)
+            *reinterpret_cast<float *>(pw.rec & ~3ull) = lane(vy4, (int)(pw.rec & 3));
+        else {
+            const int r0 = a.tl.rec_off[slot], ntr = a.tl.rec_off[slot + 1] - r0;
+            float *sm = a.tl.seis + a.tl.seis_off[slot] + (long long)(nt - 1) * ntr;
+            for (int e = tr0; e < tr1; e++) {
+                const int pk = __ldg(a.tl.rpt + e);
+                const int ri = pk & 0xffff, rj = pk >> 16;
+                if (rj == j && ri >= i0 && ri < i0 + 4) sm[__ldg(a.tl.rid + e)] = lane(vy4, ri - i0);
+            }
         }
     }
 
@@ -489,8 +705,8 @@ __global__ void __launch_bounds__(BX *BY, (FLAGS & (VF_CORR | VF_HESS)) ? VSTEP_
     v_step(StepArgs a, int nt_off)
 {
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    v_body<FDO, FLAGS, P2>(a, nt_off, 1 + 4 * (blockIdx.x * BX + threadIdx.x), j, blockIdx.z,
-                           ((j - 1) / BY) * gridDim.x + blockIdx.x);
+    v_body<FDO, FLAGS, P2, GlobalTaps<>, false, false>(a, nt_off, 1 + 4 * (blockIdx.x * BX + threadIdx.x), j, blockIdx.z,
+                                                       ((j - 1) / BY) * gridDim.x + blockIdx.x);
 }
 
 /*
@@ -828,58 +1044,26 @@ __device__ __forceinline__ void s_body(const StepArgs &a, int nt_off, int i0, in
     const float dhi = (L > 0) ? a.dhi_visc : a.dhi_el;
     const bool in_pml = a.fw > 0 && (i0 <= a.fw || i0 + 3 >= a.nx - a.fw + 1 || (!a.free_surf && j <= a.fw) ||
                                      j >= a.ny - a.fw + 1);
-    float4 vyx4 = make_float4(0.f, 0.f, 0.f, 0.f), vyy4 = vyx4;
+    float dx[4], dy[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const int i = i0 + k;
-        float vyx, vyy;
 #pragma unroll
         for (int m = 1; m <= H; m++) {
             float tx = a.hc[m] * (xs[4 * NL + k + m] - xs[4 * NL + k - m + 1]);
             float ty = a.hc[m] * (get(ys[H - 1 + m], k) - get(ys[H - m], k));
-            if (m == 1) { vyx = tx; vyy = ty; }
-            else { vyx = vyx + tx; vyy = vyy + ty; }
+            if (m == 1) { dx[k] = tx; dy[k] = ty; }
+            else { dx[k] = dx[k] + tx; dy[k] = dy[k] + ty; }
         }
-        vyx = vyx * dhi;
-        vyy = vyy * dhi;
-        const int fw = a.fw;
-        if (in_pml && i <= a.nx) {
-            if (i <= fw) {
-                float *p = a.psi_sxx + so + (long long)(j - 1) * 2 * fw + (i - 1);
-                float ps = __ldg(a.pml.b_x_half + i) * *p + __ldg(a.pml.a_x_half + i) * vyx;
-                *p = ps;
-                vyx = vyx / __ldg(a.pml.K_x_half + i) + ps;
-            }
-            if (i >= a.nx - fw + 1) {
-                const int h1 = i - a.nx + 2 * fw;
-                float *p = a.psi_sxx + so + (long long)(j - 1) * 2 * fw + (h1 - 1);
-                float ps = __ldg(a.pml.b_x_half + h1) * *p + __ldg(a.pml.a_x_half + h1) * vyx;
-                *p = ps;
-                vyx = vyx / __ldg(a.pml.K_x_half + h1) + ps;
-            }
-            if (!a.free_surf && j <= fw) {
-                float *p = a.psi_syy + so + (long long)(j - 1) * pitch + (col0 + k);
-                if (L > 0) {
-                    float ps = __ldg(a.pml.b_y + j) * *p + __ldg(a.pml.a_y + j) * vyy;
-                    *p = ps;
-                    vyy = vyy / __ldg(a.pml.K_y + j) + ps;
-                } else {
-                    float ps = __ldg(a.pml.b_y_half + j) * *p + __ldg(a.pml.a_y_half + j) * vyy;
-                    *p = ps;
-                    vyy = vyy / __ldg(a.pml.K_y_half + j) + ps;
-                }
-            }
-            if (j >= a.ny - fw + 1) {
-                const int h1 = j - a.ny + 2 * fw;
-                float *p = a.psi_syy + so + (long long)(h1 - 1) * pitch + (col0 + k);
-                float ps = __ldg(a.pml.b_y_half + h1) * *p + __ldg(a.pml.a_y_half + h1) * vyy;
-                *p = ps;
-                vyy = vyy / __ldg(a.pml.K_y_half + h1) + ps;
-            }
-        }
-        set(vyx4, k, vyx);
-        set(vyy4, k, vyy);
+        dx[k] = dx[k] * dhi;
+        dy[k] = dy[k] * dhi;
     }
+    if (in_pml) {                            /* the viscoelastic top strip takes the full-grid profiles */
+        const CpmlAxis cx{a.pml.K_x_half, a.pml.a_x_half, a.pml.b_x_half},
+            cy{a.pml.K_y_half, a.pml.a_y_half, a.pml.b_y_half}, cf{a.pml.K_y, a.pml.a_y, a.pml.b_y};
+        cpml4(a, i0, j, nvalid, dx, dy, a.psi_sxx + so + (long long)(j - 1) * 2 * a.fw, a.psi_syy + so, cx,
+              L > 0 ? cf : cy, cy);
+    }
+    const float4 vyx4 = make_float4(dx[0], dx[1], dx[2], dx[3]), vyy4 = make_float4(dy[0], dy[1], dy[2], dy[3]);
 
     /* ---- stress and memory-variable update ---- */
     if (L == 0) {
@@ -1020,12 +1204,39 @@ __device__ __forceinline__ void s_body(const StepArgs &a, int nt_off, int i0, in
     }
 }
 
+/* Receiver samples of step nt (seismo_ssg.c:17-27) by the blocks of one extra
+ * block row of the stress launch, in the receivers' own order: the velocity
+ * kernel's threads then carry no receiver state, and the samples are taken
+ * beside the stress update instead of at the end of the velocity update
+ * (a chain of four dependent loads). */
+__device__ __forceinline__ void sample_block(const StepArgs &a, int nt_off)
+{
+    const int nt = *a.nt_base + nt_off, slot = blockIdx.z, step = gridDim.x * blockDim.x * blockDim.y;
+    const int r0 = a.tl.rec_off[slot], ntr = a.tl.rec_off[slot + 1] - r0;
+    float *sm = a.tl.seis + a.tl.seis_off[slot] + (long long)(nt - 1) * ntr;
+    const float *vy = a.vy + (long long)slot * a.slot_stride;
+    int r = (blockIdx.x * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
+    int pt = r < ntr ? __ldg(a.tl.rec_pt + r0 + r) : 0;
+    pdl_wait();                              /* velocities of this step are complete */
+    pdl_trigger();
+    if (nt > a.nt_last) return;
+    while (r < ntr) {
+        sm[r] = vy[pt];
+        r += step;
+        if (r < ntr) pt = __ldg(a.tl.rec_pt + r0 + r);
+    }
+}
+
 /* one thread block = 128 x blockDim.y points of one shot slot (grid z);
  * blockDim.y = 8, 4 or 2 (a shorter block lifetime shortens the last,
  * partly idle wave of a launch) */
 template <int FDO, int L, int FLAGS>
 __global__ void __launch_bounds__(BX *BY, SSTEP_MIN_BLOCKS) s_step(StepArgs a, int nt_off)
 {
+    if (!(FLAGS & (SF_CORR | SF_HESS | SF_PARAMS)) && a.tl.samp_by > 0 && (int)blockIdx.y == a.tl.samp_by) {
+        sample_block(a, nt_off);
+        return;
+    }
     s_body<FDO, L, FLAGS>(a, nt_off, 1 + 4 * (blockIdx.x * BX + threadIdx.x), 1 + blockIdx.y * blockDim.y + threadIdx.y,
                           blockIdx.z);
 }
