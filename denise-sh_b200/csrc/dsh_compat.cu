@@ -246,6 +246,7 @@ StepArgs base_args(const float *hc)
     a.dt = DT; a.dh = DH;
     a.inv_dh = (float)(1.0 / (double)DH);
     a.rdh_d = 1.0 / (double)DH;
+    a.rdh_lo = INFINITY;
     a.dhi_el = DT / DH;
     a.dhi_visc = (float)(1.0 / (double)DH);
     a.dthalbe = (float)((double)DT / 2.0);

@@ -551,14 +551,13 @@ extern "C" dsh_ctx *dsh_create(const dsh_params *p, int device, int *status)
     if (!dh_pow2(p->dh) && p->dh >= 0x1p-20f && p->dh <= 0x1p20f) {
         ctx->rdh_h = (float)(1.0 / (double)p->dh);
         ctx->rdh_l = (float)(1.0 / (double)p->dh - (double)ctx->rdh_h);
-        ctx->rdh_lo = std::max(std::max(0x1p-100f, 0x1p-100f * p->dh), 0x1p-124f / std::fabs(ctx->rdh_l));
-        ctx->rdh_hi = std::min(0x1p100f, 0x1p100f * p->dh);
+        const float lo = std::max(std::max(0x1p-100f, 0x1p-100f * p->dh), 0x1p-124f / std::fabs(ctx->rdh_l));
         int differ = 1;
         rdh_check<<<(1 << 23) / 256, 256>>>(p->dh, ctx->rdh_h, ctx->rdh_l, ctx->d_status);
         if (cudaMemcpy(&differ, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
             cudaMemset(ctx->d_status, 0, sizeof(int)) != cudaSuccess)
             return bail(DSH_ERR_CUDA);
-        ctx->rdh_on = !differ && ctx->rdh_lo < ctx->rdh_hi;
+        if (!differ) ctx->rdh_lo = lo;
     }
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(DSH_ERR_CUDA);
     memset(&ctx->stats, 0, sizeof(ctx->stats));
@@ -789,9 +788,11 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
         return ((j - 1) / BY) * gx + (i - 1) / (4 * BX);
     };
     struct Grp { int i, j, tile; std::vector<int> members; };
-    /* appends groups (sorted by tile, stable) and fills the tile table of slot s */
+    /* appends groups (sorted by tile, row and column) and fills the tile table of slot s */
     auto emit = [&](std::vector<Grp> &gs, int *tab) {
-        std::stable_sort(gs.begin(), gs.end(), [](const Grp &x, const Grp &y) { return x.tile < y.tile; });
+        std::stable_sort(gs.begin(), gs.end(), [](const Grp &x, const Grp &y) {
+            return x.tile != y.tile ? x.tile < y.tile : x.j != y.j ? x.j < y.j : x.i < y.i;
+        });
         size_t k = 0;
         for (int t = 0; t <= T; t++) {
             while (k < gs.size() && gs[k].tile < t) k++;
@@ -865,7 +866,11 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
                 rec_pt.push_back(pt_of(i, j));
                 ent.push_back({tile_of(i, j), r});
             }
-            std::stable_sort(ent.begin(), ent.end(), [](auto &x, auto &y) { return x.first < y.first; });
+            std::stable_sort(ent.begin(), ent.end(), [&](auto &x, auto &y) {
+                const int ix = sh.recpos[x.second], jx = sh.recpos[sh.ntr + x.second];
+                const int iy = sh.recpos[y.second], jy = sh.recpos[sh.ntr + y.second];
+                return x.first != y.first ? x.first < y.first : jx != jy ? jx < jy : ix < iy;
+            });
             ctx->ntr_b[s] = sh.ntr;
             seis_off[s] = nseis;
             out_off[s] = nseis;
@@ -884,6 +889,20 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
         }
     }
     rec_off[S] = (int)rec_pt.size();
+    /* row spans of the lists: part of the captured launches, so they only
+       grow (to multiples of 32 rows) and a batch inside them keeps the graphs */
+    bool grown = false;
+    auto span = [&](int *r, const std::vector<int> &pk, int a, int b) {
+        for (int e = a; e < b; e++) {
+            const int j = (int)((unsigned)pk[e] >> 16), lo = j / 32 * 32, hi = lo + 31;
+            if (r[1] < r[0]) { r[0] = lo; r[1] = hi; grown = true; }
+            if (lo < r[0]) { r[0] = lo; grown = true; }
+            if (hi > r[1]) { r[1] = hi; grown = true; }
+        }
+    };
+    span(ctx->rows_f, gpk, fgrp_off[0], fgrp_off[S]);
+    span(ctx->rows_a, gpk, agrp_off[0], agrp_off[S]);
+    span(ctx->rows_r, rpk, 0, (int)rpk.size());
     ctx->geo_max_groups = ctx->geo_max_members = ctx->geo_max_ntr = 0;
     for (int s = 0; s < nb; s++) {
         ctx->geo_max_groups = std::max(ctx->geo_max_groups, fgrp_off[s + 1] - fgrp_off[s]);
@@ -927,7 +946,7 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
     const long long F = 3LL * (S + 1) + 3LL * S * (T + 1) + 2LL * S * (FT + 1);
     const long long maxlen = (long long)std::max({grp_pt.size(), grp_beg.size(), src_id.size(), rec_pt.size(),
                                                   gpk.size(), rpk.size(), rid.size(), fvids.size()}) + 1;
-    bool realloc = false;
+    bool realloc = grown;
     if (F + 9 * maxlen > ctx->geo_cap) {
         cudaFree(ctx->d_geo);
         ctx->d_geo = nullptr;
@@ -1060,7 +1079,7 @@ StepArgs step_args(dsh_ctx *ctx, Pass pass)
     a.dt = p.dt; a.dh = p.dh;
     a.inv_dh = (float)(1.0 / (double)p.dh);
     a.pml_k1 = ctx->pml_k1;
-    a.rdh_on = ctx->rdh_on; a.rdh_h = ctx->rdh_h; a.rdh_l = ctx->rdh_l; a.rdh_lo = ctx->rdh_lo; a.rdh_hi = ctx->rdh_hi;
+    a.rdh_h = ctx->rdh_h; a.rdh_l = ctx->rdh_l; a.rdh_lo = ctx->rdh_lo;
     a.rdh_d = 1.0 / (double)p.dh;
     a.dhi_el = p.dt / p.dh;
     a.dhi_visc = (float)(1.0 / (double)p.dh);
@@ -1122,6 +1141,14 @@ StepArgs step_args(dsh_ctx *ctx, Pass pass)
         a.tl.sig_ss = p.nt; a.tl.sig_ts = 1;
         a.tl.sample = (pass == P_FWD_HESS || pass == P_RECOMP) ? 0 : 1;
     }
+    const int *rows = pass == P_ADJ ? ctx->rows_a : ctx->rows_f, *rr = ctx->rows_r;
+    a.tl.row0 = rows[0];
+    a.tl.row1 = rows[1];
+    if (a.tl.sample && rr[1] >= rr[0]) {
+        a.tl.row0 = rows[1] < rows[0] ? rr[0] : std::min(rows[0], rr[0]);
+        a.tl.row1 = rows[1] < rows[0] ? rr[1] : std::max(rows[1], rr[1]);
+    }
+    if (!a.tl.on) { a.tl.row0 = 1; a.tl.row1 = 0; }
     switch (pass) {
     case P_FWD_PLAIN:
         break;
@@ -1325,6 +1352,8 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
     if (sa.tl.on && sa.tl.sample) {          /* the stress launch samples the receivers (sample_block) */
         sa.tl.samp_by = (int)grid.y;
         sa.tl.sample = 0;
+        sa.tl.row0 = ctx->rows_f[0];
+        sa.tl.row1 = ctx->rows_f[1];
         grid.y += 1;
     }
     dim3 vgrid, vblock;

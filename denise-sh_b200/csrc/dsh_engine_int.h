@@ -6,6 +6,7 @@
 #include "dsh_setup.h"
 
 #include <chrono>
+#include <cmath>
 #include <map>
 #include <thread>
 #include <vector>
@@ -46,8 +47,7 @@ struct dsh_ctx {
     float *sums = nullptr;                /* sum_u, sum_rho, out_a, out_b (dense pitched) */
     float hc[7] = {0}, bip[4] = {0}, bjm[4] = {0}, cip[4] = {0}, cjm[4] = {0}, cnorm[2] = {0};
     int pml_k1 = 0;                       /* every CPML stretching K is 1 */
-    int rdh_on = 0;                       /* div_dh's product form gives RN(x / DH) (see dsh_kernels.cuh) */
-    float rdh_h = 0.0f, rdh_l = 0.0f, rdh_lo = 0.0f, rdh_hi = 0.0f;
+    float rdh_h = 0.0f, rdh_l = 0.0f, rdh_lo = INFINITY;   /* div_dh's product form (StepArgs) */
     int model_set = 0;
     float *fwd = nullptr;
     long long fwd_slot_stride = 0, fwd_step_stride = 0;
@@ -63,6 +63,8 @@ struct dsh_ctx {
     int *d_fgrp_off, *d_agrp_off, *d_grp_pt, *d_grp_beg, *d_src_id, *d_rec_off, *d_rec_pt;
     int *d_ftile, *d_atile, *d_rtile, *d_gpk, *d_rpk, *d_rid;
     int ntiles = 0, fused_inject = 0;
+    int rows_f[2] = {1, 0}, rows_a[2] = {1, 0}, rows_r[2] = {1, 0};   /* row spans of the forward sources, adjoint sources
+                                                                        and receivers seen so far (empty: 1, 0) */
     int *d_fvoff = nullptr, *d_avoff = nullptr, *d_fvids = nullptr;   /* fused-tile injection lists */
     int *d_gsid = nullptr;                /* per source group: its source if it has one, else -1 */
     int fvg_ntiles = 0;

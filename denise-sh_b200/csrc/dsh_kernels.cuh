@@ -78,6 +78,7 @@ struct TileLists {
     const long long *seis_off;
     int ntiles;
     int ntx;                     /* list tiles along x: ceil(nx / 128); tile of (i, j) = ((j-1)/8)*ntx + (i-1)/128 */
+    int row0, row1;              /* span of the rows (1-based) in which the lists of this pass may hold a point */
     int samp_by;                 /* kernel pair: block row of the stress launch that samples the receivers, 0: none */
     int on;                      /* fused path active (all positions inside the grid) */
     int sample;
@@ -99,8 +100,8 @@ struct StepArgs {
     long long slot_stride;       /* floats between consecutive shot slots */
     float hc[7];
     float dt, dh, inv_dh, dhi_el, dhi_visc, dthalbe;
-    int rdh_on, pml_k1;          /* div_dh's product form proven for this DH; every CPML K is 1 */
-    float rdh_h, rdh_l, rdh_lo, rdh_hi;
+    int pml_k1;                  /* every CPML K is 1 */
+    float rdh_h, rdh_l, rdh_lo;  /* div_dh: RN(1/DH), RN(1/DH - rdh_h), lower end of the product form's range */
     double rdh_d;                /* 1 / DH */
     PmlCoef pml;
     /* per-slot state (slot 0 base; slot s at + s*slot_stride) */
@@ -295,14 +296,14 @@ __device__ __forceinline__ long long store_idx(int s, int mod) { return s < mod 
 __device__ __forceinline__ void stay_in_branch() { asm volatile("" ::: "memory"); }
 
 /* x / DH: when DH is a power of two the product with the exact reciprocal is
- * the same correctly rounded value, so P2 kernels multiply.  Otherwise, when
- * the host set rdh_on, the division by a divisor known in advance of
+ * the same correctly rounded value, so P2 kernels multiply.  Otherwise, the
+ * division by a divisor known in advance of
  * Brisebarre, Muller and Raina (IEEE Trans. Comput. 53(8), 2004):
  *   q = RN(x zh + RN(x zl)),  zh = RN(1/DH), zl = RN(1/DH - zh),
  * a product and a fused multiply-add.  Whether it gives RN(x/DH) depends only
  * on x's significand as long as nothing under- or overflows, so dsh_create
- * compares it with the division for all 2^23 significands (rdh_check) and
- * rdh_lo <= |x| <= rdh_hi keeps RN(x zl) and q in the normal range; zeros
+ * compares it with the division for all 2^23 significands (rdh_check; rdh_lo
+ * is infinite where they differ) and rdh_lo <= |x| <= RDH_HI keeps RN(x zl) and q in the normal range; zeros
  * keep their sign.  Everything else (the tiny values ahead of a wavefront
  * above all) takes div_dh_double.  Per step of a 2000 x 800 grid, FDORDER 8,
  * DH 0.6 the divisions cost 5.5 us, these 0.6. */
@@ -315,9 +316,10 @@ __device__ __forceinline__ void stay_in_branch() { asm volatile("" ::: "memory")
 __device__ __forceinline__ float div_dh_double(float x, const StepArgs &a)
 {
     const double xd = (double)x, dh = (double)a.dh, q = xd * a.rdh_d;
-    return isfinite(x) ? (float)__fma_rn(__fma_rn(-q, dh, xd), a.rdh_d, q) : x;
+    return isfinite(x) && x != 0.0f ? (float)__fma_rn(__fma_rn(-q, dh, xd), a.rdh_d, q) : x;
 }
 
+constexpr float RDH_HI = 0x1p100f;       /* and 2^-20 <= DH <= 2^20 */
 __device__ __forceinline__ float rdh_product(float x, float zh, float zl) { return __fmaf_rn(x, zh, __fmul_rn(x, zl)); }
 
 template <bool P2>
@@ -325,8 +327,7 @@ __device__ __forceinline__ float div_dh(float x, const StepArgs &a)
 {
     if (P2) return x * a.inv_dh;
     const float ax = fabsf(x);
-    if (a.rdh_on && ((ax >= a.rdh_lo && ax <= a.rdh_hi) || ax == 0.0f))
-        return ax == 0.0f ? x : rdh_product(x, a.rdh_h, a.rdh_l);
+    if (ax >= a.rdh_lo && ax <= RDH_HI) return rdh_product(x, a.rdh_h, a.rdh_l);
     stay_in_branch();
     return div_dh_double(x, a);
 }
@@ -340,11 +341,11 @@ __device__ __forceinline__ void div4_dh(float *x, const StepArgs &a)
         for (int k = 0; k < 4; k++) x[k] = x[k] * a.inv_dh;
         return;
     }
-    bool in = a.rdh_on != 0;
+    bool in = true;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const float ax = fabsf(x[k]);
-        in = in && ((ax >= a.rdh_lo && ax <= a.rdh_hi) || ax == 0.0f);
+        in = in && ((ax >= a.rdh_lo && ax <= RDH_HI) || ax == 0.0f);
     }
     if (in) {
 #pragma unroll
@@ -498,62 +499,100 @@ struct SharedTaps {
 
 /* What the lists of a tile hold for a thread's four points, found before the
  * previous kernel's results are waited for (the lists and signals do not
- * depend on them): at most one source point with one source (its signal at
- * this step in sig, the point in inj), at most one receiver (the address of
- * its sample, the point in the two low bits).  A thread with more walks the
- * lists after the update (INJ_MANY, REC_MANY). */
-constexpr int INJ_NONE = 0, INJ_ONE = 1, INJ_MANY = 5;
+ * depend on them): the points with one source (bits 0-3 of inj) and their
+ * signals at this step, and at most one receiver (the address of its sample,
+ * the point in the two low bits).  Several sources at a point, more than NI
+ * source points or several receivers: the thread walks the lists after the
+ * update (INJ_MANY, REC_MANY). */
+constexpr int INJ_MANY = 16;
 constexpr unsigned long long REC_MANY = 1;           /* no address: sample addresses are 4-byte aligned and > 4 */
+template <int NI>
 struct PointWork {
     int inj;
-    float sig;
+    float sig[NI];
     unsigned long long rec;
 };
 
-/* The lanes of a warp (one row j, four points each) read 32 list entries at a
- * time and pass on those of their row.  Each thread walking its tile's lists
- * by itself after the update cost a chain of five dependent loads per step in
- * the tiles that hold a source or a receiver: 160 x 80, FDORDER 4, one
- * source and 32 receivers: 1.3 us of 11.1 us per step. */
-template <bool SAMPLE>
-__device__ __forceinline__ void point_lists(const StepArgs &a, int nt, int i0, int j, int slot, int tg0, int tg1, int tr0,
-                                            int tr1, PointWork *w)
+/* First of the entries of row j, sorted by column, that lies at or right of
+ * column i, among 32 list entries held one per lane (lanes of row j in m):
+ * lane number, or one past the row's last */
+__device__ __forceinline__ int list_lower(unsigned mask, unsigned m, int col, int i)
 {
-    w->inj = INJ_NONE;
-    w->sig = 0.0f;
+    int a = __ffs(m) - 1, b = 32 - __clz(m);
+#pragma unroll
+    for (int it = 0; it < 6; it++) {
+        const int mid = (a + b) >> 1, v = __shfl_sync(mask, col, mid & 31);
+        if (a < b) {
+            if (v < i) a = mid + 1;
+            else b = mid;
+        }
+    }
+    return a;
+}
+
+/* The lanes of a warp (one row j, four points each) read 32 list entries at a
+ * time and search those of their row, which the host sorted by column.  Each
+ * thread walking its tile's lists by itself after the update cost a chain of
+ * five dependent loads per step in the tiles that hold a source or receiver
+ * (160 x 80, FDORDER 4, one source, 32 receivers: 1.3 us of 11.1 us per step),
+ * and as many turns as the tile has receivers in the adjoint (8 shots of 160 x
+ * 80, 48 receivers as sources: 22.6 us for the velocity launch, 7.5 us now). */
+template <int NI, bool SAMPLE>
+__device__ __forceinline__ void point_lists(const StepArgs &a, int nt, int i0, int j, int slot, int tile, PointWork<NI> *w)
+{
+    w->inj = 0;
     w->rec = 0;
-    if (tg0 >= tg1 && !(SAMPLE && tr0 < tr1)) return;    /* the tile's ranges: the same in all lanes */
+#pragma unroll
+    for (int q = 0; q < NI; q++) w->sig[q] = 0.0f;
+    /* rows outside the span of all lists (the same answer in all lanes) read nothing */
+    if (j < a.tl.row0 || j > a.tl.row1) return;
     const int ln = threadIdx.x & 31;
     const int live = min(32, (a.nx - (i0 - 4 * ln)) / 4 + 1);      /* lanes inside the grid */
     const unsigned mask = live >= 32 ? 0xffffffffu : (1u << live) - 1;
-    for (int base = tg0; base < tg1; base += live) {
-        const int pk = base + ln < tg1 ? __ldg(a.tl.gpt + base + ln) : 0;
-        const int sl = base + ln < tg1 ? __ldg(a.tl.gsid + base + ln) : 0;
-        const float *sig = a.tl.sig + a.tl.sig_off[slot] + (long long)(min(nt, a.nt_last) - 1) * a.tl.sig_ts;
-        unsigned m = __ballot_sync(mask, (int)((unsigned)pk >> 16) == j);
-        while (m) {
-            const int l = __ffs(m) - 1;
-            m &= m - 1;
-            const int k = (__shfl_sync(mask, pk, l) & 0xffff) - i0, sid = __shfl_sync(mask, sl, l);
-            if (k < 0 || k > 3) continue;
-            if (w->inj != INJ_NONE || sid < 0) { w->inj = INJ_MANY; continue; }
-            w->inj = INJ_ONE + k;
-            w->sig = __ldg(sig + (long long)sid * a.tl.sig_ss);
+    const int *go = a.tl.goff + (long long)slot * (a.tl.ntiles + 1) + tile;
+    const int g0 = __ldg(go), g1 = __ldg(go + 1);
+    const float *sig = a.tl.sig + a.tl.sig_off[slot] + (long long)(min(nt, a.nt_last) - 1) * a.tl.sig_ts;
+    int r0 = 0, r1 = 0;
+    if (SAMPLE && a.tl.sample) {
+        const int *ro = a.tl.roff + (long long)slot * (a.tl.ntiles + 1) + tile;
+        r0 = __ldg(ro);
+        r1 = __ldg(ro + 1);
+    }
+    for (int base = g0; base < g1; base += live) {
+        const bool in = ln < live && base + ln < g1;
+        const int pk = in ? __ldg(a.tl.gpt + base + ln) : 0;
+        const int sl = in ? __ldg(a.tl.gsid + base + ln) : 0;
+        const unsigned m = __ballot_sync(mask, (int)((unsigned)pk >> 16) == j);
+        if (!m) continue;
+        const int col = pk & 0xffff, f = list_lower(mask, m, col, i0), end = 32 - __clz(m);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int k = __shfl_sync(mask, col, (f + q) & 31) - i0, sid = __shfl_sync(mask, sl, (f + q) & 31);
+            if (f + q >= end || k > 3) continue;
+            if (sid < 0 || (NI < 4 && w->inj)) { w->inj |= INJ_MANY; continue; }
+            const float v = __ldg(sig + (long long)sid * a.tl.sig_ss);
+            w->inj |= 1 << k;
+            if (NI < 4) w->sig[0] = v;
+            else
+#pragma unroll
+                for (int e = 0; e < NI; e++) w->sig[e] = e == k ? v : w->sig[e];
         }
     }
     if (!SAMPLE) return;
-    for (int base = tr0; base < tr1; base += live) {
-        const int pk = base + ln < tr1 ? __ldg(a.tl.rpt + base + ln) : 0;
-        unsigned m = __ballot_sync(mask, (int)((unsigned)pk >> 16) == j);
-        while (m) {
-            const int l = __ffs(m) - 1;
-            m &= m - 1;
-            const int k = (__shfl_sync(mask, pk, l) & 0xffff) - i0;
-            if (k < 0 || k > 3) continue;
+    for (int base = r0; base < r1; base += live) {
+        const bool in = ln < live && base + ln < r1;
+        const int pk = in ? __ldg(a.tl.rpt + base + ln) : 0;
+        const int id = in ? __ldg(a.tl.rid + base + ln) : 0;
+        const unsigned m = __ballot_sync(mask, (int)((unsigned)pk >> 16) == j);
+        if (!m) continue;
+        const int col = pk & 0xffff, f = list_lower(mask, m, col, i0), end = 32 - __clz(m);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int k = __shfl_sync(mask, col, (f + q) & 31) - i0, rid = __shfl_sync(mask, id, (f + q) & 31);
+            if (f + q >= end || k > 3) continue;
             if (w->rec) { w->rec = REC_MANY; continue; }
-            const int r0 = a.tl.rec_off[slot], ntr = a.tl.rec_off[slot + 1] - r0;
-            const float *sm = a.tl.seis + a.tl.seis_off[slot] + (long long)(nt - 1) * ntr + __ldg(a.tl.rid + base + l);
-            w->rec = (unsigned long long)sm | (unsigned)k;
+            const int o = a.tl.rec_off[slot], ntr = a.tl.rec_off[slot + 1] - o;
+            w->rec = (unsigned long long)(a.tl.seis + a.tl.seis_off[slot] + (long long)(nt - 1) * ntr + rid) | (unsigned)k;
         }
     }
 }
@@ -580,22 +619,13 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
     float4 g4, h4, f4;
     if (FLAGS & VF_CORR) g4 = ld4(a.grho + so + drow + col0);
     if (FLAGS & VF_HESS) h4 = ld4(a.hrho + so + drow + col0);
-    int tg0 = 0, tg1 = 0, tr0 = 0, tr1 = 0;
-    if (a.tl.on) {
-        const int *go = a.tl.goff + (long long)slot * (a.tl.ntiles + 1) + tile;
-        tg0 = __ldg(go); tg1 = __ldg(go + 1);
-        if (SAMPLE && a.tl.sample) {
-            const int *ro = a.tl.roff + (long long)slot * (a.tl.ntiles + 1) + tile;
-            tr0 = __ldg(ro); tr1 = __ldg(ro + 1);
-        }
-    }
     if (FLAGS & VF_CORR) {                   /* stored forward acceleration of step NT-nt+1 (the address
                                                 clamped so that a step beyond the pass stays in range) */
         const long long k = store_idx(max(a.nt_total - nt, 0), a.fwd_mod);
         f4 = ldcs4(a.fwd + (long long)slot * a.fwd_slot_stride + k * a.fwd_step_stride + drow + col0);
     }
-    PointWork pw;
-    point_lists<SAMPLE>(a, nt, i0, j, slot, tg0, tg1, tr0, tr1, &pw);
+    PointWork<(FLAGS & VF_ADJOINT) ? 4 : 1> pw;
+    point_lists<(FLAGS & VF_ADJOINT) ? 4 : 1, SAMPLE>(a, nt, i0, j, slot, tile, &pw);
     pdl_wait();                              /* stresses of the previous step are complete */
     pdl_trigger();
 
@@ -648,11 +678,9 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
     }
 
     /* ---- fused injection (sources in order per point) and sampling ---- */
-    if (pw.inj == INJ_ONE + 0) vy4.x = vy4.x + pw.sig;
-    else if (pw.inj == INJ_ONE + 1) vy4.y = vy4.y + pw.sig;
-    else if (pw.inj == INJ_ONE + 2) vy4.z = vy4.z + pw.sig;
-    else if (pw.inj == INJ_ONE + 3) vy4.w = vy4.w + pw.sig;
-    else if (pw.inj == INJ_MANY) {
+    if (pw.inj & INJ_MANY) {
+        const int *go = a.tl.goff + (long long)slot * (a.tl.ntiles + 1) + tile;
+        const int tg0 = __ldg(go), tg1 = __ldg(go + 1);
         for (int g = tg0; g < tg1; g++) {
             const int pk = __ldg(a.tl.gpt + g);
             const int gi = pk & 0xffff, gj = pk >> 16;
@@ -664,6 +692,12 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
                 set_lane(vy4, gi - i0, v);
             }
         }
+    } else if (pw.inj) {
+        constexpr bool ALL = (FLAGS & VF_ADJOINT) != 0;
+        if (pw.inj & 1) vy4.x = vy4.x + pw.sig[0];
+        if (pw.inj & 2) vy4.y = vy4.y + pw.sig[ALL ? 1 : 0];
+        if (pw.inj & 4) vy4.z = vy4.z + pw.sig[ALL ? 2 : 0];
+        if (pw.inj & 8) vy4.w = vy4.w + pw.sig[ALL ? 3 : 0];
     }
     if (SAMPLE && pw.rec) {
         if (pw.rec != REC_MANY)
@@ -671,6 +705,8 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
         else {
             const int r0 = a.tl.rec_off[slot], ntr = a.tl.rec_off[slot + 1] - r0;
             float *sm = a.tl.seis + a.tl.seis_off[slot] + (long long)(nt - 1) * ntr;
+            const int *ro = a.tl.roff + (long long)slot * (a.tl.ntiles + 1) + tile;
+            const int tr0 = __ldg(ro), tr1 = __ldg(ro + 1);
             for (int e = tr0; e < tr1; e++) {
                 const int pk = __ldg(a.tl.rpt + e);
                 const int ri = pk & 0xffff, rj = pk >> 16;

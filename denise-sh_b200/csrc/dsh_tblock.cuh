@@ -64,6 +64,14 @@ __host__ __device__ inline long long tb_smem_bytes(const TbGeom &g)
     return 4LL * (TB_FIELDS * (long long)g.ew * g.eh + TB_MAX_GRP * (3 + TB_MAX_MEM) + 2LL * TB_MAX_REC + 2);
 }
 
+/* d / K of a strip point (K = 1 unless the model stretches its strips) */
+__device__ __forceinline__ float over_k(float d, const float *K, bool k_one)
+{
+    if (k_one) return d;
+    stay_in_branch();
+    return d / __ldg(K);
+}
+
 template <int FDO, bool P2>
 __global__ void __launch_bounds__(TB_THREADS) tb_fwd(StepArgs a, TbGeom geo, int n_first, int ksteps)
 {
@@ -72,7 +80,7 @@ __global__ void __launch_bounds__(TB_THREADS) tb_fwd(StepArgs a, TbGeom geo, int
     const int slot = blockIdx.z;
     const long long so = (long long)slot * a.slot_stride;
     const int nx = a.nx, ny = a.ny, fw = a.fw, pitch = a.pitch;
-    const bool top = !a.free_surf;
+    const bool top = !a.free_surf, k_one = a.pml_k1 != 0;
     const int ox = 1 + blockIdx.x * geo.tw, oy = 1 + blockIdx.y * geo.th;      /* first own point */
     const int ox1 = min(ox + geo.tw - 1, nx), oy1 = min(oy + geo.th - 1, ny);  /* last own point */
     const int gx0 = ox - geo.g, gy0 = oy - geo.g, ew = geo.ew, eh = geo.eh;
@@ -193,22 +201,22 @@ __global__ void __launch_bounds__(TB_THREADS) tb_fwd(StepArgs a, TbGeom geo, int
                     if (i <= fw) {
                         const float ps = __ldg(a.pml.b_x + i) * pvx[p] + __ldg(a.pml.a_x + i) * sxy_x;
                         pvx[p] = ps;
-                        sxy_x = sxy_x / __ldg(a.pml.K_x + i) + ps;
+                        sxy_x = over_k(sxy_x, a.pml.K_x + i, k_one) + ps;
                     } else if (i >= nx - fw + 1) {
                         const int h1 = i - nx + 2 * fw;
                         const float ps = __ldg(a.pml.b_x + h1) * pvx[p] + __ldg(a.pml.a_x + h1) * sxy_x;
                         pvx[p] = ps;
-                        sxy_x = sxy_x / __ldg(a.pml.K_x + h1) + ps;
+                        sxy_x = over_k(sxy_x, a.pml.K_x + h1, k_one) + ps;
                     }
                     if (top && j <= fw) {
                         const float ps = __ldg(a.pml.b_y + j) * pvy[p] + __ldg(a.pml.a_y + j) * syy_y;
                         pvy[p] = ps;
-                        syy_y = syy_y / __ldg(a.pml.K_y + j) + ps;
+                        syy_y = over_k(syy_y, a.pml.K_y + j, k_one) + ps;
                     } else if (j >= ny - fw + 1) {
                         const int h1 = j - ny + 2 * fw;
                         const float ps = __ldg(a.pml.b_y + h1) * pvy[p] + __ldg(a.pml.a_y + h1) * syy_y;
                         pvy[p] = ps;
-                        syy_y = syy_y / __ldg(a.pml.K_y + h1) + ps;
+                        syy_y = over_k(syy_y, a.pml.K_y + h1, k_one) + ps;
                     }
                 }
                 const float b = br[p];
@@ -260,22 +268,22 @@ __global__ void __launch_bounds__(TB_THREADS) tb_fwd(StepArgs a, TbGeom geo, int
                     if (i <= fw) {
                         const float ps = __ldg(a.pml.b_x_half + i) * psx[p] + __ldg(a.pml.a_x_half + i) * vyx;
                         psx[p] = ps;
-                        vyx = vyx / __ldg(a.pml.K_x_half + i) + ps;
+                        vyx = over_k(vyx, a.pml.K_x_half + i, k_one) + ps;
                     } else if (i >= nx - fw + 1) {
                         const int h1 = i - nx + 2 * fw;
                         const float ps = __ldg(a.pml.b_x_half + h1) * psx[p] + __ldg(a.pml.a_x_half + h1) * vyx;
                         psx[p] = ps;
-                        vyx = vyx / __ldg(a.pml.K_x_half + h1) + ps;
+                        vyx = over_k(vyx, a.pml.K_x_half + h1, k_one) + ps;
                     }
                     if (top && j <= fw) {
                         const float ps = __ldg(a.pml.b_y_half + j) * psy[p] + __ldg(a.pml.a_y_half + j) * vyy;
                         psy[p] = ps;
-                        vyy = vyy / __ldg(a.pml.K_y_half + j) + ps;
+                        vyy = over_k(vyy, a.pml.K_y_half + j, k_one) + ps;
                     } else if (j >= ny - fw + 1) {
                         const int h1 = j - ny + 2 * fw;
                         const float ps = __ldg(a.pml.b_y_half + h1) * psy[p] + __ldg(a.pml.a_y_half + h1) * vyy;
                         psy[p] = ps;
-                        vyy = vyy / __ldg(a.pml.K_y_half + h1) + ps;
+                        vyy = over_k(vyy, a.pml.K_y_half + h1, k_one) + ps;
                     }
                 }
                 const float nsx = sxy[p] + ui[p] * vyx, nsz = syz[p] + uj[p] * vyy;
