@@ -41,6 +41,7 @@ static void build_tmaps(dsh_ctx *ctx);
 namespace {
 
 
+constexpr long long SPLIT_MIN_POINTS = 1 << 17;   /* slot_split */
 constexpr int RED_BLOCKS = 296;        /* 2 x 148 SMs for reductions */
 constexpr int RED_THREADS = 256;
 
@@ -477,6 +478,10 @@ extern "C" dsh_ctx *dsh_create(const dsh_params *p, int device, int *status)
     ctx->st = ctx->own_st;
     for (int k = 0; k < 4; k++) cudaEventCreate(&ctx->ev[k]);
     if (cudaEventCreateWithFlags(&ctx->ev_wait, cudaEventDisableTiming) != cudaSuccess) return bail(DSH_ERR_CUDA);
+    if (cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess)
+        return bail(DSH_ERR_CUDA);
     const int nx = p->nx, ny = p->ny, L = p->l, fw = p->fw;
     ctx->H = p->fdorder / 2;
     ctx->hy = ctx->H;
@@ -587,6 +592,9 @@ extern "C" int dsh_destroy(dsh_ctx *ctx)
     cudaFree(ctx->d_taper_box); cudaFree(ctx->d_taper_shot); cudaFree(ctx->d_tmap);
     for (int k = 0; k < 4; k++) if (ctx->ev[k]) cudaEventDestroy(ctx->ev[k]);
     if (ctx->ev_wait) cudaEventDestroy(ctx->ev_wait);
+    if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
+    if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+    if (ctx->st2) cudaStreamDestroy(ctx->st2);
     if (ctx->own_st) cudaStreamDestroy(ctx->own_st);
     delete ctx;
     return DSH_OK;
@@ -1329,6 +1337,21 @@ static int launch_fused_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chu
 static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chunk, long long *nlaunch)
 {
     if (use_fused(ctx, pass)) return launch_fused_chunk(ctx, pass, nb, nsteps_in_chunk, nlaunch);
+/* Two independent halves of a launch's shot slots (the kernel pair with fused
+ * injection): first slot of the second half, 0 when the slots stay together.
+ * The velocity launch is bound by latency and instruction issue, the stress
+ * launch by DRAM; on two streams the velocity launch of one half overlaps the
+ * stress launch of the other, and no launch's last, partly idle wave leaves
+ * the device idle. */
+static int slot_split(const dsh_ctx *ctx, const VPick &vp, int nb)
+{
+    static const char *env = getenv("DSH_SLOT_SPLIT");
+    if (vp.code != 0 || nb < 2 || !ctx->fused_inject) return 0;
+    const long long pts = (long long)ctx->p.nx * ctx->p.ny * (nb / 2);
+    const bool on = env ? atoi(env) != 0 : pts >= SPLIT_MIN_POINTS;
+    return on ? nb / 2 : 0;
+}
+
     const dsh_params &p = ctx->p;
     int vflags = 0, sflags = 0;
     switch (pass) {
@@ -1370,25 +1393,39 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
     cfg.dynamicSmemBytes = 0;
     cfg.stream = ctx->st;
     static const bool use_pdl = getenv("DSH_NO_PDL") == nullptr;
-    for (int k = 0; k < nsteps_in_chunk; k++) {
-        int off = k;
-        void *args[2] = {&sa, &off};
-        cfg.attrs = (use_pdl && k > 0) ? &attr : nullptr;
-        cfg.numAttrs = (use_pdl && k > 0) ? 1 : 0;
-        cfg.gridDim = vgrid;
-        cfg.blockDim = vblock;
-        CK(cudaLaunchKernelExC(&cfg, (const void *)vk, args));
-        cfg.gridDim = grid;
-        cfg.blockDim = block;
-        if (!sa.tl.on) {
-            void *iargs[2] = {&ia, &off};
-            CK(cudaLaunchKernel((const void *)inject_sample, dim3(nb), dim3(128), iargs, 0, ctx->st));
-            *nlaunch += 1;
+    const int half = slot_split(ctx, vp, nb);
+    if (half) {
+        CK(cudaEventRecord(ctx->ev_fork, ctx->st));
+        CK(cudaStreamWaitEvent(ctx->st2, ctx->ev_fork, 0));
+    }
+    for (int part = 0; part < (half ? 2 : 1); part++) {
+        const int s0 = part ? half : 0, ns = half ? (part ? nb - half : half) : nb;
+        cfg.stream = part ? ctx->st2 : ctx->st;
+        for (int k = 0; k < nsteps_in_chunk; k++) {
+            int off = launch_word(k, s0);
+            void *args[2] = {&sa, &off};
+            cfg.attrs = (use_pdl && k > 0) ? &attr : nullptr;
+            cfg.numAttrs = (use_pdl && k > 0) ? 1 : 0;
+            cfg.gridDim = vgrid;
+            if (half) cfg.gridDim.z = (unsigned)ns;
+            cfg.blockDim = vblock;
+            CK(cudaLaunchKernelExC(&cfg, (const void *)vk, args));
+            cfg.gridDim = dim3(grid.x, grid.y, (unsigned)ns);
+            cfg.blockDim = block;
+            if (!sa.tl.on) {
+                void *iargs[2] = {&ia, &off};
+                CK(cudaLaunchKernel((const void *)inject_sample, dim3(nb), dim3(128), iargs, 0, ctx->st));
+                *nlaunch += 1;
+            }
+            cfg.attrs = use_pdl ? &attr : nullptr;
+            cfg.numAttrs = use_pdl ? 1 : 0;
+            CK(cudaLaunchKernelExC(&cfg, (const void *)sk, args));
+            *nlaunch += 2;
         }
-        cfg.attrs = use_pdl ? &attr : nullptr;
-        cfg.numAttrs = use_pdl ? 1 : 0;
-        CK(cudaLaunchKernelExC(&cfg, (const void *)sk, args));
-        *nlaunch += 2;
+    }
+    if (half) {
+        CK(cudaEventRecord(ctx->ev_join, ctx->st2));
+        CK(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
     }
     advance_step<<<1, 1, 0, ctx->st>>>(ctx->d_nt, nsteps_in_chunk);
     *nlaunch += 1;

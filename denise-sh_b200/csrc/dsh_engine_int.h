@@ -23,6 +23,8 @@ struct dsh_ctx {
     int dev = 0;
     cudaStream_t st = nullptr;
     cudaStream_t own_st = nullptr;
+    cudaStream_t st2 = nullptr;           /* second half of the shot slots (slot_split), forked from st and joined to it */
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int H = 0, hy = 0, pitch = 0, S = 1, chunk = 32;
     long long fstride = 0, dstride = 0, slot_stride = 0;
     long long o_vy, o_sxy, o_syz, o_r, o_q, o_pvxx, o_psxx, o_pvyy, o_psyy, o_state_end;

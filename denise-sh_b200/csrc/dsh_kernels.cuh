@@ -572,10 +572,12 @@ __device__ __forceinline__ void point_lists(const StepArgs &a, int nt, int i0, i
             if (sid < 0 || (NI < 4 && w->inj)) { w->inj |= INJ_MANY; continue; }
             const float v = __ldg(sig + (long long)sid * a.tl.sig_ss);
             w->inj |= 1 << k;
-            if (NI < 4) w->sig[0] = v;
-            else
+            if constexpr (NI < 4) {
+                w->sig[0] = v;
+            } else {
 #pragma unroll
                 for (int e = 0; e < NI; e++) w->sig[e] = e == k ? v : w->sig[e];
+            }
         }
     }
     if (!SAMPLE) return;
@@ -734,14 +736,21 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
     }
 }
 
+/* The launch word of v_step and s_step: the step's offset from the counter in
+ * the low 16 bits, the first shot slot of the launch in the high ones. */
+__host__ __device__ __forceinline__ int launch_word(int nt_off, int slot0) { return nt_off | (int)((unsigned)slot0 << 16); }
+__device__ __forceinline__ int word_off(int w) { return w & 0xffff; }
+__device__ __forceinline__ int word_slot(int w) { return (int)blockIdx.z + (int)((unsigned)w >> 16); }
+
 /* one thread block = 128 x blockDim.y points of one shot slot (grid z),
  * blockDim.y dividing the 8 rows of an injection / sampling list tile */
 template <int FDO, int FLAGS, bool P2>
 __global__ void __launch_bounds__(BX *BY, (FLAGS & (VF_CORR | VF_HESS)) ? VSTEP_MIN_BLOCKS : VSTEP_MIN_BLOCKS_FWD)
-    v_step(StepArgs a, int nt_off)
+    v_step(StepArgs a, int word)
 {
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    v_body<FDO, FLAGS, P2, GlobalTaps<>, false, false>(a, nt_off, 1 + 4 * (blockIdx.x * BX + threadIdx.x), j, blockIdx.z,
+    v_body<FDO, FLAGS, P2, GlobalTaps<>, false, false>(a, word_off(word), 1 + 4 * (blockIdx.x * BX + threadIdx.x), j,
+                                                       word_slot(word),
                                                        ((j - 1) / BY) * gridDim.x + blockIdx.x);
 }
 
@@ -1245,9 +1254,9 @@ __device__ __forceinline__ void s_body(const StepArgs &a, int nt_off, int i0, in
  * kernel's threads then carry no receiver state, and the samples are taken
  * beside the stress update instead of at the end of the velocity update
  * (a chain of four dependent loads). */
-__device__ __forceinline__ void sample_block(const StepArgs &a, int nt_off)
+__device__ __forceinline__ void sample_block(const StepArgs &a, int nt_off, int slot)
 {
-    const int nt = *a.nt_base + nt_off, slot = blockIdx.z, step = gridDim.x * blockDim.x * blockDim.y;
+    const int nt = *a.nt_base + nt_off, step = gridDim.x * blockDim.x * blockDim.y;
     const int r0 = a.tl.rec_off[slot], ntr = a.tl.rec_off[slot + 1] - r0;
     float *sm = a.tl.seis + a.tl.seis_off[slot] + (long long)(nt - 1) * ntr;
     const float *vy = a.vy + (long long)slot * a.slot_stride;
@@ -1267,14 +1276,14 @@ __device__ __forceinline__ void sample_block(const StepArgs &a, int nt_off)
  * blockDim.y = 8, 4 or 2 (a shorter block lifetime shortens the last,
  * partly idle wave of a launch) */
 template <int FDO, int L, int FLAGS>
-__global__ void __launch_bounds__(BX *BY, SSTEP_MIN_BLOCKS) s_step(StepArgs a, int nt_off)
+__global__ void __launch_bounds__(BX *BY, SSTEP_MIN_BLOCKS) s_step(StepArgs a, int word)
 {
     if (!(FLAGS & (SF_CORR | SF_HESS | SF_PARAMS)) && a.tl.samp_by > 0 && (int)blockIdx.y == a.tl.samp_by) {
-        sample_block(a, nt_off);
+        sample_block(a, word_off(word), word_slot(word));
         return;
     }
-    s_body<FDO, L, FLAGS>(a, nt_off, 1 + 4 * (blockIdx.x * BX + threadIdx.x), 1 + blockIdx.y * blockDim.y + threadIdx.y,
-                          blockIdx.z);
+    s_body<FDO, L, FLAGS>(a, word_off(word), 1 + 4 * (blockIdx.x * BX + threadIdx.x), 1 + blockIdx.y * blockDim.y + threadIdx.y,
+                          word_slot(word));
 }
 
 /* Source injection then receiver sampling for one step, one block per slot
