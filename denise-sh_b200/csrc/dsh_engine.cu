@@ -588,7 +588,7 @@ extern "C" int dsh_destroy(dsh_ctx *ctx)
     cudaFree(ctx->ckpt); cudaFree(ctx->shadow);
     cudaFree(ctx->d_geo); cudaFree(ctx->d_offs); cudaFree(ctx->d_sig); cudaFree(ctx->d_seis); cudaFree(ctx->d_res);
     cudaFree(ctx->d_obs); cudaFree(ctx->d_tmp); cudaFree(ctx->d_out); cudaFree(ctx->d_nt); cudaFree(ctx->d_part); cudaFree(ctx->d_l2);
-    cudaFree(ctx->d_wemax); cudaFree(ctx->d_gq); cudaFree(ctx->d_flags);
+    cudaFree(ctx->d_wemax); cudaFree(ctx->d_gq); cudaFree(ctx->d_flags); cudaFree(ctx->d_tb);
     cudaFree(ctx->d_taper_box); cudaFree(ctx->d_taper_shot); cudaFree(ctx->d_tmap);
     for (int k = 0; k < 4; k++) if (ctx->ev[k]) cudaEventDestroy(ctx->ev[k]);
     if (ctx->ev_wait) cudaEventDestroy(ctx->ev_wait);
@@ -911,12 +911,15 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
     span(ctx->rows_f, gpk, fgrp_off[0], fgrp_off[S]);
     span(ctx->rows_a, gpk, agrp_off[0], agrp_off[S]);
     span(ctx->rows_r, rpk, 0, (int)rpk.size());
-    ctx->geo_max_groups = ctx->geo_max_members = ctx->geo_max_ntr = 0;
+    ctx->geo_max_groups = ctx->geo_max_members = ctx->geo_max_ntr = ctx->geo_max_src = ctx->geo_max_adj_members = 0;
     for (int s = 0; s < nb; s++) {
         ctx->geo_max_groups = std::max(ctx->geo_max_groups, fgrp_off[s + 1] - fgrp_off[s]);
         for (int g = fgrp_off[s]; g < fgrp_off[s + 1]; g++)
             ctx->geo_max_members = std::max(ctx->geo_max_members, grp_beg[g + 1] - grp_beg[g]);
         ctx->geo_max_ntr = std::max(ctx->geo_max_ntr, ctx->ntr_b[s]);
+        ctx->geo_max_src = std::max(ctx->geo_max_src, grp_beg[fgrp_off[s + 1]] - grp_beg[fgrp_off[s]]);
+        for (int g = agrp_off[s]; g < agrp_off[s + 1]; g++)
+            ctx->geo_max_adj_members = std::max(ctx->geo_max_adj_members, grp_beg[g + 1] - grp_beg[g]);
     }
 
     /* fused step: per slot and 128 x 16 tile, the groups whose point lies in
@@ -1334,9 +1337,6 @@ static int launch_fused_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chu
     return DSH_OK;
 }
 
-static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chunk, long long *nlaunch)
-{
-    if (use_fused(ctx, pass)) return launch_fused_chunk(ctx, pass, nb, nsteps_in_chunk, nlaunch);
 /* Two independent halves of a launch's shot slots (the kernel pair with fused
  * injection): first slot of the second half, 0 when the slots stay together.
  * The velocity launch is bound by latency and instruction issue, the stress
@@ -1352,6 +1352,9 @@ static int slot_split(const dsh_ctx *ctx, const VPick &vp, int nb)
     return on ? nb / 2 : 0;
 }
 
+static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chunk, long long *nlaunch)
+{
+    if (use_fused(ctx, pass)) return launch_fused_chunk(ctx, pass, nb, nsteps_in_chunk, nlaunch);
     const dsh_params &p = ctx->p;
     int vflags = 0, sflags = 0;
     switch (pass) {
@@ -1477,6 +1480,8 @@ static int persistent_grid(dsh_ctx *ctx, Pass pass, int nb)
     return tiles <= (long long)per_sm * nsm ? (int)tiles : 0;
 }
 
+static int ensure_flags(dsh_ctx *ctx, long long n);
+
 static int run_persistent(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, int grid)
 {
     const dsh_params &p = ctx->p;
@@ -1486,16 +1491,8 @@ static int run_persistent(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, in
     set_int_kernel<<<1, 1, 0, ctx->st>>>(ctx->d_nt, n0);
     /* completion flags of the tiles (velocity and stress step per tile and slot) */
     const long long nflags = 2LL * grid;
-    if (nflags > ctx->flags_cap) {
-        cudaFree(ctx->d_flags);
-        ctx->d_flags = nullptr;
-        ctx->flags_cap = 0;
-        if (cudaMalloc(&ctx->d_flags, (size_t)nflags * sizeof(unsigned)) != cudaSuccess) {
-            cudaGetLastError();
-            return DSH_ERR_OOM;
-        }
-        ctx->flags_cap = nflags;
-    }
+    const int rc = ensure_flags(ctx, nflags);
+    if (rc != DSH_OK) return rc;
     CK(cudaMemsetAsync(ctx->d_flags, 0, (size_t)nflags * sizeof(unsigned), ctx->st));
     unsigned *bar = ctx->d_flags;
     void *args[3] = {&sa, &count, &bar};
@@ -1537,34 +1534,75 @@ static int run_cluster(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, const
     return DSH_OK;
 }
 
-/* Small elastic grids, plain forward modelling: k time steps per launch of
- * tb_fwd (dsh_tblock.cuh), each CTA advancing its tile and a recomputed halo
- * in shared memory.  On by DSH_TBLOCK=1 or the autotuner's choice; false
- * when it does not apply (viscoelastic, FDORDER > 8, positions outside the
- * grid, more sources or receivers per shot than its lists hold). */
-static bool tblock_cfg(dsh_ctx *ctx, Pass pass, int nb, TbCfg *cfg)
+/* Small elastic grids: a whole pass in one launch of tb_pass (dsh_tblock.cuh),
+ * one tile per SM, several steps between two exchanges of the tiles' halos.
+ * Serves every pass but the Hessian's.  false when it does not apply
+ * (viscoelastic, FDORDER > 8, positions outside the grid, more sources or
+ * receivers per shot than its lists hold, tiles that do not fit the SMs). */
+static bool tblock_cfg(dsh_ctx *ctx, Pass pass, int nb, TbProblem *pb, TbCfg *cfg)
 {
-    static const int env = env_flag("DSH_TBLOCK");
-    const bool on = ctx->sel_tblock >= 0 ? ctx->sel_tblock != 0 : env != 0;
+    static const char *env = getenv("DSH_TBLOCK");
+    /* a variable that picks or shapes another step kernel asks for that one */
+    static const bool other = [] {
+        for (const char *v : {"DSH_FUSED", "DSH_VSTAGE", "DSH_VTMA", "DSH_VROWS", "DSH_PERSIST", "DSH_CLUSTER", "DSH_SROWS",
+                              "DSH_VBROWS", "DSH_L2_STREAM", "DSH_SLOT_SPLIT"})
+            if (getenv(v)) return true;
+        return false;
+    }();
+    const bool on = ctx->sel_tblock >= 0 ? ctx->sel_tblock != 0 : env ? atoi(env) != 0 : !other;
     const dsh_params &p = ctx->p;
-    if (!on || pass != P_FWD_PLAIN || !ctx->fused_inject || p.l != 0 || p.fdorder > 8) return false;
-    TbProblem pb;
-    pb.fdorder = p.fdorder; pb.p2 = dh_pow2(p.dh) ? 1 : 0; pb.nx = p.nx; pb.ny = p.ny; pb.fw = p.fw; pb.nb = nb;
-    pb.max_groups = ctx->geo_max_groups; pb.max_members = ctx->geo_max_members;
-    pb.max_receivers = ctx->geo_max_ntr;
-    return tb_config(pb, cfg);
+    if (!on || pass == P_FWD_HESS || !ctx->fused_inject || p.l != 0 || p.fdorder > 8) return false;
+    if (ctx->sel_fused > 0 || ctx->sel_staged > 0 || ctx->sel_persist > 0) return false;     /* another variant is chosen */
+    pb->fdorder = p.fdorder; pb->p2 = dh_pow2(p.dh) ? 1 : 0; pb->nx = p.nx; pb->ny = p.ny; pb->fw = p.fw; pb->nb = nb;
+    pb->mode = pass == P_ADJ ? TB_ADJ : (pass == P_FWD_STORE || pass == P_RECOMP) ? TB_STORE : TB_FWD;
+    pb->max_entries = pass == P_ADJ ? ctx->geo_max_ntr : ctx->geo_max_src;
+    pb->max_members = pass == P_ADJ ? ctx->geo_max_adj_members : ctx->geo_max_members;
+    pb->max_receivers = pass == P_ADJ ? 0 : ctx->geo_max_ntr;
+    /* unless asked for, only with two steps or more between two exchanges (us
+       per step against the pair's: 160 x 80, FDORDER 4, k 4: 2.2 and 4.1; 500 x
+       200: 2.9 and 4.6; 700 x 280: 3.6 and 5.1; FDORDER 8, k 2: 3.5 and 4.3, 4.3
+       and 4.9; with one step the pair is faster: 1000 x 300 6.8 and 5.4, 700 x
+       280, FDORDER 8: 7.0 and 6.0) */
+    pb->min_k = ctx->sel_tblock > 0 || env ? 1 : 2;
+    return tb_config(*pb, cfg);
 }
 
-static int run_tblock(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, const TbCfg &cfg)
+static int ensure_flags(dsh_ctx *ctx, long long n)
 {
-    const dsh_params &p = ctx->p;
+    if (n > ctx->flags_cap) {
+        cudaFree(ctx->d_flags);
+        ctx->d_flags = nullptr;
+        ctx->flags_cap = 0;
+        if (cudaMalloc(&ctx->d_flags, (size_t)n * sizeof(unsigned)) != cudaSuccess) {
+            cudaGetLastError();
+            return DSH_ERR_OOM;
+        }
+        ctx->flags_cap = n;
+    }
+    return DSH_OK;
+}
+
+static int run_tblock(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, const TbProblem &pb, const TbCfg &cfg)
+{
     StepArgs sa = step_args(ctx, pass);
     sa.nslots = nb;
-    long long nl = 0;
-    const cudaError_t e = tb_launch(cfg, p.fdorder, dh_pow2(p.dh), sa, n0, count, nb, ctx->st, &nl);
-    ctx->launches += nl;
-    CK(e);
-    ctx->state_b = 0;
+    int rc = ensure_flags(ctx, cfg.tiles);
+    if (rc != DSH_OK) return rc;
+    const long long need = 2LL * nb * TB_XFIELDS * ctx->dstride;
+    if (need > ctx->tb_cap) {
+        cudaFree(ctx->d_tb);
+        ctx->d_tb = nullptr;
+        ctx->tb_cap = 0;
+        if (cudaMalloc(&ctx->d_tb, (size_t)need * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            return DSH_ERR_OOM;
+        }
+        ctx->tb_cap = need;
+    }
+    CK(cudaMemsetAsync(ctx->d_flags, 0, (size_t)cfg.tiles * sizeof(unsigned), ctx->st));
+    CK(tb_launch(cfg, pb, sa, TbExchange{ctx->d_tb, ctx->d_flags}, n0, count, ctx->st));
+    ctx->launches += 1;
+    if (pass != P_RECOMP) ctx->state_b = 0;
     return DSH_OK;
 }
 
@@ -1576,7 +1614,8 @@ static int run_steps(dsh_ctx *ctx, Pass pass, int nb, int n0, int count)
     ClCfg ccfg;
     if (cluster_cfg(ctx, pass, nb, &ccfg)) return run_cluster(ctx, pass, nb, n0, count, ccfg);
     TbCfg tcfg;
-    if (tblock_cfg(ctx, pass, nb, &tcfg)) return run_tblock(ctx, pass, nb, n0, count, tcfg);
+    TbProblem tpb;
+    if (tblock_cfg(ctx, pass, nb, &tpb, &tcfg)) return run_tblock(ctx, pass, nb, n0, count, tpb, tcfg);
     if (const int grid = persistent_grid(ctx, pass, nb)) return run_persistent(ctx, pass, nb, n0, count, grid);
     const int K = std::min(ctx->chunk, count);
     const int nfull = count / K, rem = count % K;
@@ -2193,7 +2232,8 @@ extern "C" int dsh_autotune(dsh_ctx *ctx, const dsh_shot *shots, int nshots, int
         if (v == 3 && !persistent_grid(ctx, P_FWD_PLAIN, nb)) continue;
         if (v == 4 && !cluster_cfg(ctx, P_FWD_PLAIN, nb, &ccfg)) continue;
         TbCfg tcfg;
-        if (v == 5 && !tblock_cfg(ctx, P_FWD_PLAIN, nb, &tcfg)) continue;
+        TbProblem tpb;
+        if (v == 5 && !tblock_cfg(ctx, P_FWD_PLAIN, nb, &tpb, &tcfg)) continue;
         for (int rep = 0; rep < 2; rep++) {            /* first round warms up (graphs, lazy loading) */
             if ((rc = zero_slots(ctx, nb, false)) != DSH_OK) break;
             CK(cudaEventRecord(e0, ctx->st));

@@ -79,9 +79,12 @@ struct dsh_ctx {
     unsigned *d_bar = nullptr;            /* (unused spare words after the status word) */
     unsigned *d_flags = nullptr;          /* tile completion flags of the persistent launch */
     long long flags_cap = 0;
+    float *d_tb = nullptr;                /* exchange buffers of the temporally blocked pass */
+    long long tb_cap = 0;
     double *d_part = nullptr, *d_l2 = nullptr;
     unsigned *d_wemax = nullptr;
     std::vector<int> ntr_b;
+    int geo_max_src = 0, geo_max_adj_members = 0;                   /* forward sources, receivers at one point */
     int geo_max_groups = 0, geo_max_members = 0, geo_max_ntr = 0;   /* last batch, per slot: forward source
                                                                        points, sources at one point, receivers */
     int lnorm = 2;                        /* misfit norm of the residual (dsh_set_misfit) */

@@ -1,32 +1,50 @@
-/* Instantiations, launch shape and launches of the temporally blocked
- * forward-modelling kernel (dsh_tblock.cuh), FDORDER 2..8. */
+/* Instantiations, launch shape and launch of the temporally blocked pass of
+ * small elastic grids (dsh_tblock.cuh), FDORDER 2..8. */
 #include <algorithm>
 #include <cstdlib>
 
 #include "dsh_tb.h"
 
 namespace dsh {
-using TbFn = void (*)(StepArgs, TbGeom, int, int);
+using TbFn = void (*)(StepArgs, TbGeom, TbExchange, int, int);
 
-template <bool P2>
-static TbFn tb_pick(int fdo)
+template <int FDO, bool P2, int MAXT>
+static TbFn tb_mode(int mode)
+{
+    return mode == TB_ADJ     ? tb_pass<FDO, P2, TB_ADJ, MAXT>
+           : mode == TB_STORE ? tb_pass<FDO, P2, TB_STORE, MAXT>
+                              : tb_pass<FDO, P2, TB_FWD, MAXT>;
+}
+template <bool P2, int MAXT>
+static TbFn tb_pick(int fdo, int mode)
 {
     switch (fdo) {
-    case 2: return tb_fwd<2, P2>;
-    case 4: return tb_fwd<4, P2>;
-    case 6: return tb_fwd<6, P2>;
-    case 8: return tb_fwd<8, P2>;
+    case 2: return tb_mode<2, P2, MAXT>(mode);
+    case 4: return tb_mode<4, P2, MAXT>(mode);
+    case 6: return tb_mode<6, P2, MAXT>(mode);
+    case 8: return tb_mode<8, P2, MAXT>(mode);
     default: return nullptr;
     }
 }
 
-static TbFn tb_fn(int fdo, bool p2) { return p2 ? tb_pick<true>(fdo) : tb_pick<false>(fdo); }
+static TbFn tb_fn(const TbProblem &pb, int nthr)
+{
+    if (nthr <= TB_FEW_THREADS)
+        return pb.p2 ? tb_pick<true, TB_FEW_THREADS>(pb.fdorder, pb.mode) : tb_pick<false, TB_FEW_THREADS>(pb.fdorder, pb.mode);
+    return pb.p2 ? tb_pick<true, TB_MAX_THREADS>(pb.fdorder, pb.mode) : tb_pick<false, TB_MAX_THREADS>(pb.fdorder, pb.mode);
+}
+
+static int env_int(const char *name, int lo, int hi)
+{
+    const char *e = getenv(name);
+    const int v = e ? atoi(e) : 0;
+    return v >= lo && v <= hi ? v : 0;
+}
 
 bool tb_config(const TbProblem &pb, TbCfg *cfg)
 {
-    const TbFn fk = tb_fn(pb.fdorder, pb.p2 != 0);
-    if (!fk || pb.nb < 1 || pb.nx < 1 || pb.ny < 1 || pb.nx > 0xffff || pb.ny > 0x7fff) return false;
-    if (pb.max_groups > TB_MAX_GRP || pb.max_members > TB_MAX_MEM || pb.max_receivers > TB_MAX_REC) return false;
+    if (pb.fdorder < 2 || pb.fdorder > 8 || (pb.fdorder & 1) || pb.nb < 1 || pb.nx < 1 || pb.ny < 1 || pb.nx > 0xffff || pb.ny > 0x7fff) return false;
+    if (pb.max_entries > TB_MAX_ENT || pb.max_members > TB_MAX_MEM || pb.max_receivers > TB_MAX_REC) return false;
     if (pb.fw > 0 && (pb.nx < 2 * pb.fw || pb.ny < 2 * pb.fw)) return false;
     int dev = 0, maxsm = 0, nsm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -35,48 +53,44 @@ bool tb_config(const TbProblem &pb, TbCfg *cfg)
         cudaGetLastError();
         return false;
     }
-    const int R = pb.fdorder - 1;
-    int k = pb.fdorder == 2 ? 8 : pb.fdorder == 4 ? 4 : pb.fdorder == 6 ? 3 : 2;
-    if (const char *e = getenv("DSH_TB_STEPS")) {
-        const int v = atoi(e);
-        if (v >= 1 && v <= 64) k = v;
-    }
-    int rows = 0;                                    /* tile height pinned by DSH_TB_ROWS */
-    if (const char *e = getenv("DSH_TB_ROWS")) {
-        const int v = atoi(e);
-        if (v >= 1 && v <= 256) rows = v;
-    }
+    if ((long long)pb.nx * pb.ny * pb.nb > 4LL * TB_MAX_THREADS * nsm) return false;     /* more vectors than threads */
+    const int H = pb.fdorder / 2, R = pb.fdorder - 1;
+    const int kmax = pb.fdorder == 2 ? 8 : pb.fdorder == 4 ? 4 : pb.fdorder == 6 ? 3 : 2;
+    const int kpin = env_int("DSH_TB_STEPS", 1, 64), rows = env_int("DSH_TB_ROWS", 1, 256);
+    double best = 0.0;
     TbCfg c;
-    c.geo.tw = 32;
-    auto shape = [&](int th, int kk) {
-        c.geo.th = th;
-        c.geo.g = kk * R;
-        c.geo.ew = c.geo.tw + 2 * c.geo.g;
-        c.geo.eh = c.geo.th + 2 * c.geo.g;
-        return tb_smem_bytes(c.geo) <= maxsm;
+    auto consider = [&](int tw, int th, int k) {
+        TbGeom g;
+        g.tw = tw; g.th = th; g.k = k;
+        g.gy = k * R; g.gx = (g.gy + 3) / 4 * 4;
+        g.nv = (tw + 2 * g.gx) / 4; g.eh = th + 2 * g.gy;
+        g.ntx = (pb.nx + tw - 1) / tw; g.nty = (pb.ny + th - 1) / th;
+        g.nthr = (g.nv * g.eh + 31) / 32 * 32;
+        g.nent = std::max(4, (pb.max_entries + 3) / 4 * 4);
+        g.nrec = std::max(4, (pb.max_receivers + 3) / 4 * 4);
+        const long long tiles = (long long)g.ntx * g.nty * pb.nb;
+        const long long bytes = 4LL * tb_smem(g, H, pb.mode).total;
+        if (g.nthr > TB_MAX_THREADS || tiles > nsm || bytes > maxsm) return false;
+        /* per step one vector of a thread, per round the exchange (us; 160 x 80: 1.3 + 2.8 / k, 500 x 200: 2.1 + 2.8 / k) */
+        const double step = 0.7 + 0.0021 * g.nthr, t = step + 2.8 / k;
+        if (best == 0.0 || t < best) {
+            best = t;
+            c.geo = g;
+            c.tiles = (int)tiles;
+            c.smem = (size_t)bytes;
+        }
+        return true;
     };
-    /* tile height: the smallest multiple of 8 rows (up to 64) for which every
-       tile of every slot runs at once, one CTA per SM (a second wave, or SMs
-       holding two tiles beside SMs holding one, would double the time of the
-       slowest SM); 16 rows where no height does */
-    int th = 16;
-    if (rows) {
-        th = rows;
-    } else {
-        const int ntx = (pb.nx + c.geo.tw - 1) / c.geo.tw;
-        for (int t = 8; t <= 64; t += 8)
-            if ((long long)ntx * ((pb.ny + t - 1) / t) * pb.nb <= nsm && shape(t, k)) {
-                th = t;
-                break;
+    for (int tw = 32; tw <= 64; tw += 32)
+        for (int th = rows ? rows : 8; th <= (rows ? rows : 128); th += 8) {
+            if (kpin) {
+                for (int k = kpin; k >= 1 && !consider(tw, th, k); k--) {}
+            } else {
+                for (int k = kmax; k >= pb.min_k; k--) consider(tw, th, k);
             }
-    }
-    for (; k >= 1; k--)
-        if (shape(th, k)) break;
-    if (k < 1) return false;
-    c.k = k;
-    c.ntx = (pb.nx + c.geo.tw - 1) / c.geo.tw;
-    c.nty = (pb.ny + c.geo.th - 1) / c.geo.th;
-    c.smem = (size_t)tb_smem_bytes(c.geo);
+        }
+    if (best == 0.0) return false;
+    const TbFn fk = tb_fn(pb, c.geo.nthr);
     /* the opt-in maximum, not this problem's size: contexts of other sizes
        may launch the same kernel concurrently */
     if (cudaFuncSetAttribute((const void *)fk, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm) != cudaSuccess) {
@@ -87,28 +101,15 @@ bool tb_config(const TbProblem &pb, TbCfg *cfg)
     return true;
 }
 
-cudaError_t tb_launch(const TbCfg &cfg, int fdorder, bool p2, const StepArgs &a, int n0, int count, int nb,
-                      cudaStream_t st, long long *nlaunch)
+cudaError_t tb_launch(const TbCfg &cfg, const TbProblem &pb, const StepArgs &a, const TbExchange &x, int n0, int count,
+                      cudaStream_t st)
 {
-    const TbFn fk = tb_fn(fdorder, p2);
-    if (!fk || cfg.k < 1) return cudaErrorInvalidValue;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)cfg.ntx, (unsigned)cfg.nty, (unsigned)nb);
-    lc.blockDim = dim3(TB_THREADS);
-    lc.dynamicSmemBytes = cfg.smem;
-    lc.stream = st;
-    static const bool use_pdl = getenv("DSH_NO_PDL") == nullptr;
-    for (int c = 0; c < count; c += cfg.k) {
-        const int ks = std::min(cfg.k, count - c);
-        lc.attrs = (use_pdl && c > 0) ? &attr : nullptr;   /* the first one follows the pass's set-up plainly */
-        lc.numAttrs = (use_pdl && c > 0) ? 1 : 0;
-        const cudaError_t e = cudaLaunchKernelEx(&lc, fk, a, cfg.geo, n0 + c, ks);
-        if (e != cudaSuccess) return e;
-        *nlaunch += 1;
-    }
-    return cudaSuccess;
+    const TbFn fk = tb_fn(pb, cfg.geo.nthr);
+    if (!fk || cfg.tiles < 1) return cudaErrorInvalidValue;
+    StepArgs sa = a;
+    TbGeom g = cfg.geo;
+    TbExchange xx = x;
+    void *args[5] = {&sa, &g, &xx, &n0, &count};
+    return cudaLaunchCooperativeKernel((const void *)fk, dim3((unsigned)cfg.tiles), dim3((unsigned)g.nthr), args, cfg.smem, st);
 }
 }  // namespace dsh

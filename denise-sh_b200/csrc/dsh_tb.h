@@ -1,5 +1,5 @@
-/* dsh_tb.h — the temporally blocked forward-modelling kernel (dsh_tblock.cuh):
- * its launch shape for a context and its launches. */
+/* dsh_tb.h — the temporally blocked pass of small elastic grids
+ * (dsh_tblock.cuh): its launch shape for a context and its launch. */
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -7,33 +7,31 @@
 #include "dsh_tblock.cuh"
 
 namespace dsh {
-/* what decides whether and how the kernel serves a plain elastic forward pass */
+/* what decides whether and how the kernel serves a pass of an elastic context */
 struct TbProblem {
-    int fdorder, p2, nx, ny, fw;
-    int nb;                      /* shot slots (grid z) */
-    int max_groups, max_members, max_receivers;   /* per slot: source points, sources at one point, receivers */
+    int fdorder, p2, mode, nx, ny, fw;
+    int nb;                      /* shot slots */
+    int min_k = 1;               /* fewest steps per round */
+    int max_entries, max_members, max_receivers;   /* per slot: sources, sources at one point, receivers */
 };
 
 struct TbCfg {
     TbGeom geo;
-    int k = 0;                   /* time steps per launch at most */
-    int ntx = 0, nty = 0;        /* own tiles along x and depth */
-    size_t smem = 0;             /* dynamic shared memory per CTA in bytes */
+    int tiles = 0;               /* blocks of the launch: tiles of all slots */
+    size_t smem = 0;             /* dynamic shared memory per block in bytes */
 };
 
-/* The launch shape on the current device: own tiles 32 points wide and as
- * few rows high (a multiple of 8, up to 64) as lets every tile of every slot
- * run at once with one CTA per SM, else 16 rows (DSH_TB_ROWS pins the
- * height); k steps per launch (FDORDER 2: 8, 4: 4, 6: 3, 8: 2; DSH_TB_STEPS
- * overrides it), k lowered until the tile fits the opt-in shared memory of
- * one CTA.  false
- * when the kernel cannot serve the problem (FDORDER > 8, more sources or
- * receivers per slot than its lists hold, NX or NY below 2 FW). */
+/* The launch shape on the current device: among tiles 32 or 64 points wide and
+ * a multiple of 8 rows high that give at most one block per SM, and k = 1 to
+ * 4 (FDORDER 2: 8, 4: 4, 6: 3, 8: 2) steps per round, the one with the least
+ * estimated time per step (tb_config in dsh_tb.cu); DSH_TB_STEPS pins k (lowered
+ * where the region does not fit a block) and DSH_TB_ROWS the height.  false
+ * when the kernel cannot serve the problem: FDORDER > 8, more sources or
+ * receivers per slot than its lists hold, NX or NY below 2 FW, or no shape
+ * with every block resident. */
 bool tb_config(const TbProblem &pb, TbCfg *cfg);
 
-/* Launches steps n0 .. n0 + count - 1 for nb slots: ceil(count / k)
- * launches of k steps (the last one the rest), each after the previous one
- * through programmatic dependent launch.  *nlaunch += the launches made. */
-cudaError_t tb_launch(const TbCfg &cfg, int fdorder, bool p2, const StepArgs &a, int n0, int count, int nb,
-                      cudaStream_t st, long long *nlaunch);
+/* Launches steps n0 .. n0 + count - 1 for the configured slots (cooperative). */
+cudaError_t tb_launch(const TbCfg &cfg, const TbProblem &pb, const StepArgs &a, const TbExchange &x, int n0, int count,
+                      cudaStream_t st);
 }  // namespace dsh

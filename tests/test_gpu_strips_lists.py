@@ -64,9 +64,10 @@ def test_forward_gradient_and_hessian(case):
     o = O.Oracle(m, "port")
     gv, gr = o.convert(su, sr)
     o.close()
-    for extra in ({}, {"ckpt_every": 17}):
+    for extra, variant in (({}, 0), ({"ckpt_every": 17}, 0), ({}, 5), ({"ckpt_every": 17}, 5), ({}, -1)):
         with dsh.Engine(dsh.make_params(max_shots=2, **kw, **extra)) as e:
             e.set_model(vs, rho, qs)
+            e.set_step_variant(variant)
             seis = e.forward(shots)
             out = e.gradient(shots, obs)
         assert all(np.array_equal(a, b) for a, b in zip(seis, ref))
@@ -126,3 +127,29 @@ def test_division_by_dh_over_magnitudes(dh):
             got = [e.field(f) for f in ("vy", "sxy", "syz")]
         assert np.array_equal(seis, ref)
         assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+def test_blocked_passes_of_two_contexts_at_once():
+    """Two small elastic contexts run their passes from two threads: launches whose blocks wait for one another."""
+    import threading
+
+    kw, vs, rho, _, shots = _case(203, 97, 10, 4, 0, 1, 0.5, 1.0, 40, seed=3)
+    engines = [dsh.Engine(dsh.make_params(max_shots=3, **kw)) for _ in range(2)]
+    out = [None, None]
+    for e in engines:
+        e.set_model(vs, rho)
+        e.set_step_variant(5)
+        e.set_wait_limits(device_polls=1 << 20)
+
+    def work(k):
+        out[k] = [engines[k].forward(shots) for _ in range(20)]
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    engines[0].set_step_variant(0)
+    ref = engines[0].forward(shots)
+    for k in range(2):
+        engines[k].close()
+        assert out[k] is not None
+        assert all(np.array_equal(a, b) for o in out[k] for a, b in zip(o, ref))
