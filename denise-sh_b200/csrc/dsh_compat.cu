@@ -244,6 +244,7 @@ StepArgs base_args(const float *hc)
     a.fstride = G.fstride; a.dstride = G.dstride; a.slot_stride = 0;
     for (int k = 0; k <= 6; k++) a.hc[k] = hc[k];
     a.dt = DT; a.dh = DH;
+    a.one = 1.0f;
     a.inv_dh = (float)(1.0 / (double)DH);
     a.rdh_d = 1.0 / (double)DH;
     a.rdh_lo = INFINITY;

@@ -1088,6 +1088,7 @@ StepArgs step_args(dsh_ctx *ctx, Pass pass)
     a.fstride = ctx->fstride; a.dstride = ctx->dstride; a.slot_stride = ctx->slot_stride;
     for (int k = 0; k < 7; k++) a.hc[k] = ctx->hc[k];
     a.dt = p.dt; a.dh = p.dh;
+    a.one = 1.0f;
     a.inv_dh = (float)(1.0 / (double)p.dh);
     a.pml_k1 = ctx->pml_k1;
     a.rdh_h = ctx->rdh_h; a.rdh_l = ctx->rdh_l; a.rdh_lo = ctx->rdh_lo;
