@@ -887,6 +887,11 @@ def bench_batch(a, rank, world, local):
     sbytes = sum(kernel_bytes(m["params"]["l"], store=False)[1] * m["params"]["nx"] * m["params"]["ny"] *
                  len(m["shots"]) for m in models)
     s_ms = st["s_ms"][st["s_variant"]]
+    s_kernel = f"s_multi_k (one stress half-step: a launch per register class, {len(models)} models)"
+    if s_ms <= 0:      # every model advanced alone: both half-steps of a whole run, bytes per step times steps
+        sbytes = sum(sum(kernel_bytes(m["params"]["l"], store=False)) * m["params"]["nx"] * m["params"]["ny"] *
+                     len(m["shots"]) * m["params"]["nt"] for m in models)
+        s_ms, s_kernel = st["ms_total"], "v_step + s_step of every model, whole run"
     s_gbs = sbytes / (s_ms / 1e3) / 1e9
     per_model = [{"model": m["name"], "nt": m["params"]["nt"], "shots": len(m["shots"]),
                   "gpt_s": pts_model[k] / (model_ms[k] / a.steps / 1e3) / 1e9,
@@ -913,7 +918,7 @@ def bench_batch(a, rank, world, local):
                        "l2": f"wavefield state {sum((3 + 2 * m['params']['l']) * m['params']['nx'] * m['params']['ny'] * len(m['shots']) for m in models) * 4 / 1e9:.1f} GB, larger than L2",
                        "parallelism": f"models{world}"},
             "roofline": {"bound": "hbm", "achieved": s_gbs, "peak": hbm, "unit": "GB/s", "frac": s_gbs / hbm,
-                         "traffic": None, "kernel": f"s_multi_k (one stress half-step: a launch per register class, {len(models)} models)",
+                         "traffic": None, "kernel": s_kernel,
                          "bytes": sbytes, "ms_per_launch": s_ms, "peak_source": peak_kind},
             "per_model": per_model,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

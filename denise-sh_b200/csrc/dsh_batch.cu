@@ -16,6 +16,15 @@
  * steps per phase; an event after each phase gives each model's completion
  * time.
  *
+ * A model whose own launches fill the device (SOLO_MIN_POINTS grid points over
+ * its shots) is advanced alone instead, through its context's step kernels,
+ * after the others: its wavefield then mostly stays in L2 from one half-step
+ * to the next and its halves of shot slots overlap (slot_split), where the
+ * whole batch in lockstep streams every wavefield from DRAM in each half-step.
+ * Eight models of 1.8-5.8 M points (9-19 shots, FDORDER 4-8, L 0 and 2): 65 ms
+ * in lockstep, 47 ms one after the other; on two or three streams at once 51
+ * and 54.  Pinned tile shapes keep every model in the common launches.
+ *
  * Reference correspondence: every model runs the forward loop of
  * src/denise.c:1179-1346 (update_v_PML, source injection, update_s_*_PML,
  * seismo_ssg) exactly as a single-model context does; the reference itself
@@ -40,6 +49,10 @@ using namespace dsh::eng;
 namespace {
 __global__ void batch_set_counter(int *p, int v) { *p = v; }
 constexpr int CHUNK = 32;
+/* below it the common launches win: a launch pair of one model then costs more
+   than its share of theirs (15.7 ns per thousand points; single-model steps of
+   1.2 M points 13.4, of 0.6 M 16.8) */
+constexpr long long SOLO_MIN_POINTS = 3 << 18;
 }  // namespace
 
 struct dsh_batch {
@@ -64,7 +77,9 @@ struct dsh_batch {
         std::vector<long long> count;      /* per phase: entries of the group's running models */
     };
     std::vector<MapClass> cls[2][MULTI_NVAR];
-    std::vector<int> nb;                   /* shots per model of the current run */
+    std::vector<int> nb;                   /* shots per model of the current run's common launches */
+    std::vector<int> solo;                 /* shots of the models advanced alone (0: in the common launches) */
+    std::vector<cudaEvent_t> ev_solo;      /* per model: its solo run is complete */
     long long sig = -1;                    /* signature of the uploaded maps */
     long long geo = -1;                    /* sum of the models' geometry versions the graphs were made for */
     int var_v = -1, var_s = -1;            /* chosen tile-shape variants (-1: tune on next run) */
@@ -150,6 +165,8 @@ extern "C" dsh_batch *dsh_batch_create(const dsh_params *p, int nmodels, int dev
     b->phase_nt.erase(std::unique(b->phase_nt.begin(), b->phase_nt.end()), b->phase_nt.end());
     b->ev.resize(b->phase_nt.size() + 1);
     for (auto &e : b->ev) cudaEventCreate(&e);
+    b->ev_solo.resize(nmodels);
+    for (auto &e : b->ev_solo) cudaEventCreate(&e);
     b->done_ms.assign(nmodels, 0.0);
     const char *fv = getenv("DSH_BATCH_VARIANT");     /* "v,s": fixed variants, no tuning */
     if (fv && sscanf(fv, "%d,%d", &b->forced_v, &b->forced_s) != 2) b->forced_v = b->forced_s = -1;
@@ -166,6 +183,7 @@ extern "C" int dsh_batch_destroy(dsh_batch *b)
     for (dsh_ctx *c : b->ctx) dsh_destroy(c);
     cudaFree(b->d_nt); cudaFree(b->d_args); cudaFree(b->d_map);
     for (auto &e : b->ev) if (e) cudaEventDestroy(e);
+    for (auto &e : b->ev_solo) if (e) cudaEventDestroy(e);
     if (b->ev_wait) cudaEventDestroy(b->ev_wait);
     if (b->own_st) cudaStreamDestroy(b->own_st);
     delete b;
@@ -466,7 +484,13 @@ static int batch_forward(dsh_batch *b, const dsh_shot *shots, const int *nshots,
 {
     if (!b || !shots || !nshots) return DSH_ERR_PARAM;
     BK(cudaSetDevice(b->dev));
+    static const bool pinned = getenv("DSH_MULTI_MIXED") || getenv("DSH_MULTI_ARGS_DEVICE");
     b->nb.assign(nshots, nshots + b->n);
+    b->solo.assign(b->n, 0);
+    if (!pinned && b->forced_v < 0 && b->forced_s < 0)
+        for (int k = 0; k < b->n; k++)
+            if ((long long)b->p[k].nx * b->p[k].ny * nshots[k] >= SOLO_MIN_POINTS) std::swap(b->nb[k], b->solo[k]);
+    const bool common = std::any_of(b->nb.begin(), b->nb.end(), [](int n) { return n > 0; });
     std::vector<long long> first(b->n + 1, 0), out_off(b->n + 1, 0);
     for (int k = 0; k < b->n; k++) {
         if (nshots[k] < 0 || nshots[k] > b->ctx[k]->S) return DSH_ERR_PARAM;
@@ -480,12 +504,12 @@ static int batch_forward(dsh_batch *b, const dsh_shot *shots, const int *nshots,
         if (nshots[k] == 0) continue;
         if ((rc = upload_batch(c, shots + first[k], nshots[k], nullptr, nullptr, 0)) != DSH_OK) return rc;
     }
-    if ((rc = build_maps(b)) != DSH_OK) return rc;
-    if ((rc = upload_args(b)) != DSH_OK) return rc;
+    if (common && (rc = build_maps(b)) != DSH_OK) return rc;
+    if (common && (rc = upload_args(b)) != DSH_OK) return rc;
     long long geo = 0;                     /* separate-injection arguments are baked into the graphs */
     for (dsh_ctx *c : b->ctx) geo += c->geo_version;
     if (geo != b->geo) { drop_batch_graphs(b); b->geo = geo; }
-    if (b->var_v < 0 || b->var_s < 0) {
+    if (common && (b->var_v < 0 || b->var_s < 0)) {
         if ((rc = tune(b)) != DSH_OK) return rc;
     }
     for (int k = 0; k < b->n; k++)
@@ -494,8 +518,18 @@ static int batch_forward(dsh_batch *b, const dsh_shot *shots, const int *nshots,
     b->points = 0;
     BK(cudaEventRecord(b->ev[0], b->st));
     for (size_t ph = 0; ph < b->phase_nt.size(); ph++) {
-        if ((rc = run_phase(b, (int)ph)) != DSH_OK) return rc;
+        if (common && (rc = run_phase(b, (int)ph)) != DSH_OK) return rc;
         BK(cudaEventRecord(b->ev[ph + 1], b->st));
+    }
+    cudaEvent_t last = b->ev[b->phase_nt.size()];
+    for (auto it = b->order.rbegin(); it != b->order.rend(); ++it) {     /* fewest steps first, as the phases */
+        const int k = *it;
+        if (b->solo[k] == 0) continue;
+        b->ctx[k]->launches = 0;
+        if ((rc = forward_steps(b->ctx[k], b->solo[k])) != DSH_OK) return rc;
+        b->launches += b->ctx[k]->launches;
+        BK(cudaEventRecord(b->ev_solo[k], b->st));
+        last = b->ev_solo[k];
     }
     for (int k = 0; k < b->n; k++) {
         if (nshots[k] == 0) continue;
@@ -510,11 +544,11 @@ static int batch_forward(dsh_batch *b, const dsh_shot *shots, const int *nshots,
     for (int k = 0; k < b->n; k++) {
         const size_t ph = std::lower_bound(b->phase_nt.begin(), b->phase_nt.end(), b->p[k].nt) - b->phase_nt.begin();
         float ms = 0;
-        cudaEventElapsedTime(&ms, b->ev[0], b->ev[ph + 1]);
+        cudaEventElapsedTime(&ms, b->ev[0], b->solo[k] ? b->ev_solo[k] : b->ev[ph + 1]);
         b->done_ms[k] = ms;
     }
     float tot = 0;
-    cudaEventElapsedTime(&tot, b->ev[0], b->ev[b->phase_nt.size()]);
+    cudaEventElapsedTime(&tot, b->ev[0], last);
     b->total_ms = tot;
     int worst = DSH_OK;
     for (int k = 0; k < b->n; k++)
@@ -542,8 +576,8 @@ extern "C" int dsh_batch_get_stats(dsh_batch *b, double *model_ms, dsh_batch_sta
         out->ms_total = b->total_ms;
         out->kernel_launches = b->launches;
         out->point_updates = b->points;
-        out->v_variant = b->var_v;
-        out->s_variant = b->var_s;
+        out->v_variant = std::max(b->var_v, 0);
+        out->s_variant = std::max(b->var_s, 0);
         for (int v = 0; v < MULTI_NVAR && v < 4; v++) {
             out->v_ms[v] = b->tune_ms[0][v];
             out->s_ms[v] = b->tune_ms[1][v];

@@ -1648,6 +1648,10 @@ static int run_steps(dsh_ctx *ctx, Pass pass, int nb, int n0, int count)
 
 static int run_pass(dsh_ctx *ctx, Pass pass, int nb) { return run_steps(ctx, pass, nb, 1, ctx->p.nt); }
 
+namespace dsh::eng {
+int forward_steps(dsh_ctx *ctx, int nb) { return run_pass(ctx, P_FWD_PLAIN, nb); }
+}  // namespace dsh::eng
+
 /* state (wavefields, memory variables, CPML memory) of slots [0, nb):
  * copy between a slab and checkpoint k */
 static int copy_state(dsh_ctx *ctx, int nb, float *dst, size_t dpitch, const float *src, size_t spitch)

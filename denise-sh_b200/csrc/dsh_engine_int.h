@@ -139,6 +139,7 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
 StepArgs step_args(dsh_ctx *ctx, Pass pass);
 InjectArgs inject_args(dsh_ctx *ctx, Pass pass);
 int zero_slots(dsh_ctx *ctx, int nb, bool accumulators);
+int forward_steps(dsh_ctx *ctx, int nb);   /* every step of a plain forward pass of slots [0, nb) */
 int copy_seis_out(dsh_ctx *ctx, int nb, float *host_out, float *dev_out);
 int check_status(dsh_ctx *ctx);
 bool dh_pow2(float dh);

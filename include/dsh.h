@@ -233,7 +233,11 @@ int dsh_residual_noalloc(int nshots, int ntr, int nt, const float *syn, const fl
  * launch for all models of a register class (the same FDORDER and L; one
  * launch holding every body for batches of more than 36 models), each thread
  * block working on one 128-point tile of one model; models leave the
- * launches once their NT is reached.  Results are bit-identical to running
+ * launches once their NT is reached.  Models of 786432 grid points or more
+ * over their shots fill the device by themselves: they are advanced one
+ * after the other through their own contexts' step kernels instead (v_ms and
+ * s_ms stay 0 in a batch of such models alone), unless the tile shape is
+ * pinned.  Results are bit-identical to running
  * each model through its own context (and so to the reference's forward
  * loop, src/denise.c:1179-1346); the reference runs one model per program.
  * Supported per model: FDORDER 4, 6, 8 and L 0 or 2 (other combinations:

@@ -129,6 +129,27 @@ def test_division_by_dh_over_magnitudes(dh):
         assert all(np.array_equal(a, b) for a, b in zip(got, want))
 
 
+def test_batch_of_small_and_large_models():
+    """A model whose launches fill the device (2 shots of 655 x 607) is advanced alone, the other with the common
+    launches; both equal their own contexts, also when the large one is left out of a later run."""
+    members = [_case(655, 607, 10, 4, 2, 1, 0.5, 1.0, 40, seed=5), _case(45, 37, 10, 8, 0, 0, 0.6, 1.0, 20, seed=6)]
+    groups = [members[0][4][:2], members[1][4]]
+    ref = []
+    for (kw, vs, rho, qs, _), shots in zip(members, groups):
+        with dsh.Engine(dsh.make_params(max_shots=3, **kw)) as e:
+            e.set_model(vs, rho, qs)
+            ref.append(e.forward(shots))
+    with dsh.Batch([dsh.make_params(max_shots=3, **m[0]) for m in members]) as b:
+        for k, m in enumerate(members):
+            b.set_model(k, *m[1:4])
+        got = b.forward(groups)
+        st = b.stats()
+        again = b.forward([[], groups[1]])
+    assert all(np.array_equal(x, y) for g, r in zip(got, ref) for x, y in zip(g, r))
+    assert st["ms_total"] == max(st["model_ms"]) and st["kernel_launches"] > 0
+    assert all(np.array_equal(x, y) for x, y in zip(again[1], ref[1]))
+
+
 def test_blocked_passes_of_two_contexts_at_once():
     """Two small elastic contexts run their passes from two threads: launches whose blocks wait for one another."""
     import threading
