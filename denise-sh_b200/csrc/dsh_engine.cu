@@ -42,6 +42,8 @@ namespace {
 
 
 constexpr long long SPLIT_MIN_POINTS = 1 << 17;   /* slot_split */
+constexpr long long GROUP_BYTES = 56LL << 20, WHOLE_BYTES = 104LL << 20;     /* slot_group */
+constexpr long long GROUP_MIN_POINTS = 3 << 18;
 constexpr int RED_BLOCKS = 296;        /* 2 x 148 SMs for reductions */
 constexpr int RED_THREADS = 256;
 
@@ -1353,7 +1355,7 @@ static int slot_split(const dsh_ctx *ctx, const VPick &vp, int nb)
     return on ? nb / 2 : 0;
 }
 
-static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chunk, long long *nlaunch)
+static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chunk, long long *nlaunch, int slot0 = 0)
 {
     if (use_fused(ctx, pass)) return launch_fused_chunk(ctx, pass, nb, nsteps_in_chunk, nlaunch);
     const dsh_params &p = ctx->p;
@@ -1403,7 +1405,7 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
         CK(cudaStreamWaitEvent(ctx->st2, ctx->ev_fork, 0));
     }
     for (int part = 0; part < (half ? 2 : 1); part++) {
-        const int s0 = part ? half : 0, ns = half ? (part ? nb - half : half) : nb;
+        const int s0 = slot0 + (part ? half : 0), ns = half ? (part ? nb - half : half) : nb;
         cfg.stream = part ? ctx->st2 : ctx->st;
         for (int k = 0; k < nsteps_in_chunk; k++) {
             int off = launch_word(k, s0);
@@ -1411,7 +1413,7 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
             cfg.attrs = (use_pdl && k > 0) ? &attr : nullptr;
             cfg.numAttrs = (use_pdl && k > 0) ? 1 : 0;
             cfg.gridDim = vgrid;
-            if (half) cfg.gridDim.z = (unsigned)ns;
+            if (half || slot0) cfg.gridDim.z = (unsigned)ns;
             cfg.blockDim = vblock;
             CK(cudaLaunchKernelExC(&cfg, (const void *)vk, args));
             cfg.gridDim = dim3(grid.x, grid.y, (unsigned)ns);
@@ -1607,6 +1609,50 @@ static int run_tblock(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, const 
     return DSH_OK;
 }
 
+/* Slots advanced together by the kernel pair: as many as keep the fields that
+ * every step touches in L2 (GROUP_BYTES); 0 when all nb nearly do
+ * (WHOLE_BYTES), or when a group would be less than a launch's worth of points.
+ * The groups then take the steps of a run one after the other, so a wavefield
+ * comes from DRAM once per run instead of in each half-step.  64 shots of 1000
+ * x 300, FDORDER 8, L 2: 285 us per step together, 246, 234, 247, 259, 263 with
+ * groups of up to 40, 56, 72, 88, 104 MB; 8 shots of 1200 x 400, L 3 (138 MB):
+ * 64.9 and 56.3; but two halves of 67 MB (8 shots of 1000 x 300) 34.0 against
+ * 30.6 together. */
+static int slot_group(const dsh_ctx *ctx, Pass pass, int nb)
+{
+    static const char *env = getenv("DSH_SLOT_GROUP_MB");
+    const dsh_params &p = ctx->p;
+    if (nb < 2 || !ctx->fused_inject || use_fused(const_cast<dsh_ctx *>(ctx), pass)) return 0;
+    if (pick_v(ctx, p.fdorder, 0, dh_pow2(p.dh)).code != 0) return 0;
+    const long long limit = env ? atoll(env) << 20 : GROUP_BYTES, pts = (long long)p.nx * p.ny;
+    const long long whole = env ? 0 : WHOLE_BYTES;
+    const int fields = 3 + 2 * p.l + (pass == P_ADJ ? 3 + 4 * p.grad_q : pass == P_FWD_HESS ? 2 : pass == P_FWD_PLAIN ? 0 : 1);
+    if (nb * 4 * pts * fields <= whole) return 0;
+    int g = (int)std::min<long long>(nb, limit / (4 * pts * fields));
+    while (g * pts < GROUP_MIN_POINTS) g++;
+    if (g >= nb) return 0;
+    const int n = (nb + g - 1) / g;
+    return (nb + n - 1) / n;
+}
+
+/* the steps of a run for one group of slots after the other; a launch lasts
+ * longer than its submission, so none are captured */
+static int run_groups(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, int group)
+{
+    if (pass != P_RECOMP) ctx->state_b = 0;
+    for (int s0 = 0; s0 < nb; s0 += group) {
+        set_int_kernel<<<1, 1, 0, ctx->st>>>(ctx->d_nt, n0);
+        ctx->launches += 1;
+        for (int done = 0; done < count; done += 0x7000) {
+            long long nl = 0;
+            const int rc = launch_step_chunk(ctx, pass, std::min(group, nb - s0), std::min(0x7000, count - done), &nl, s0);
+            if (rc != DSH_OK) return rc;
+            ctx->launches += nl;
+        }
+    }
+    return DSH_OK;
+}
+
 /* Steps n0 .. n0+count-1 of a pass: graphs of `chunk` steps replayed
  * count/chunk times, then one graph for the remaining steps. */
 static int run_steps(dsh_ctx *ctx, Pass pass, int nb, int n0, int count)
@@ -1618,6 +1664,7 @@ static int run_steps(dsh_ctx *ctx, Pass pass, int nb, int n0, int count)
     TbProblem tpb;
     if (tblock_cfg(ctx, pass, nb, &tpb, &tcfg)) return run_tblock(ctx, pass, nb, n0, count, tpb, tcfg);
     if (const int grid = persistent_grid(ctx, pass, nb)) return run_persistent(ctx, pass, nb, n0, count, grid);
+    if (const int group = slot_group(ctx, pass, nb)) return run_groups(ctx, pass, nb, n0, count, group);
     const int K = std::min(ctx->chunk, count);
     const int nfull = count / K, rem = count % K;
     const bool fused = use_fused(ctx, pass);
