@@ -25,15 +25,8 @@ namespace dsh {
 constexpr int HX = 8;            /* left halo / alignment columns */
 constexpr int BX = 32;           /* threads per block along x (4 points each) */
 constexpr int BY = 8;            /* threads per block along depth */
-#ifndef SSTEP_MIN_BLOCKS
-#define SSTEP_MIN_BLOCKS 2       /* resident stress-kernel blocks per SM the register budget targets */
-#endif
-#ifndef VSTEP_MIN_BLOCKS
-#define VSTEP_MIN_BLOCKS 3       /* resident velocity-kernel blocks per SM the register budget targets */
-#endif
 #ifndef VSTEP_MIN_BLOCKS_FWD
-#define VSTEP_MIN_BLOCKS_FWD 4   /* the same for the forward velocity kernel (no correlation), which fits
-                                    64 registers */
+#define VSTEP_MIN_BLOCKS_FWD 3   /* resident 256-thread blocks per SM of the uneven batches' velocity kernels */
 #endif
 
 /* flags of the velocity kernel */
@@ -51,6 +44,25 @@ constexpr int SF_PARAMS = 16;    /* viscoelastic: read precomputed fipjp, f, dip
 constexpr int SF_QSENS = 32;     /* with SF_STRAIN_OUT: also store the step's stress-increment
                                     sensitivities to tau (the Qs gradient's forward part) */
 constexpr int SF_CORRQ = 64;     /* with SF_CORR: accumulate the Qs-gradient correlation */
+
+/* Registers per thread of v_step and s_step in blocks of 128 threads.  Fewer
+ * registers keep more blocks on an SM (512 / 6 = 80 registers: 6 blocks, 88 and
+ * 96: 5, 128: 4) but spill.  us per step, plain / storing / adjoint: 2000 x 800,
+ * FDORDER 8, L 3: velocity 64 / 64 / 80 registers 24.9 / 31.0 / 31.7, 80 / 80 / 88:
+ * 23.0 / 28.8 / 30.6; 2 shots of 701 x 287, FDORDER 10, elastic: 9.1 / 9.3 / 8.3, 96
+ * everywhere: 6.3 / 6.8 / 7.2; FDORDER 4, 8 shots of 1000 x 300: 16.6 / 19.6 / 24.5, 72:
+ * 16.2 / 19.4 / 23.0.  Stress: 128, viscoelastic at 112 and 160 slower (adjoint of
+ * L 3 36.8 and 32.2); elastic storing and adjoint passes up to FDORDER 8 at 96:
+ * 2000 x 800 19.0 -> 18.0 and 20.9 -> 20.0 (plain 15.1 -> 15.3, FDORDER 10 adjoint 7.2
+ * -> 8.1: those keep 128). */
+__host__ __device__ constexpr int v_regs(int fdo, int flags)
+{
+    return (flags & (VF_CORR | VF_HESS)) ? (fdo <= 4 ? 72 : fdo <= 8 ? 88 : 96) : (fdo <= 4 ? 72 : fdo <= 8 ? 80 : 96);
+}
+__host__ __device__ constexpr int s_regs(int fdo, int l, int flags)
+{
+    return l == 0 && fdo <= 8 && (flags & (SF_STRAIN_OUT | SF_CORR)) ? 96 : 128;
+}
 
 struct PmlCoef {                 /* device copies, index 1..2fw */
     const float *K_x, *a_x, *b_x, *K_x_half, *a_x_half, *b_x_half;
@@ -795,8 +807,7 @@ __device__ __forceinline__ int word_slot(int w) { return (int)blockIdx.z + (int)
 /* one thread block = 128 x blockDim.y points of one shot slot (grid z),
  * blockDim.y dividing the 8 rows of an injection / sampling list tile */
 template <int FDO, int FLAGS, bool P2>
-__global__ void __launch_bounds__(BX *BY, (FLAGS & (VF_CORR | VF_HESS)) ? VSTEP_MIN_BLOCKS : VSTEP_MIN_BLOCKS_FWD)
-    v_step(StepArgs a, int word)
+__global__ void __maxnreg__(v_regs(FDO, FLAGS)) v_step(StepArgs a, int word)
 {
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
     v_body<FDO, FLAGS, P2, GlobalTaps<>, false, false>(a, word_off(word), 1 + 4 * (blockIdx.x * BX + threadIdx.x), j,
@@ -1331,7 +1342,7 @@ __device__ __forceinline__ void sample_block(const StepArgs &a, int nt_off, int 
  * blockDim.y = 8, 4 or 2 (a shorter block lifetime shortens the last,
  * partly idle wave of a launch) */
 template <int FDO, int L, int FLAGS>
-__global__ void __launch_bounds__(BX *BY, SSTEP_MIN_BLOCKS) s_step(StepArgs a, int word)
+__global__ void __maxnreg__(s_regs(FDO, L, FLAGS)) s_step(StepArgs a, int word)
 {
     if (!(FLAGS & (SF_CORR | SF_HESS | SF_PARAMS)) && a.tl.samp_by > 0 && (int)blockIdx.y == a.tl.samp_by) {
         sample_block(a, word_off(word), word_slot(word));
