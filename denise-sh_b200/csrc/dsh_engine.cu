@@ -180,9 +180,58 @@ struct EpiArgs {
     long long slot_stride;
     float *ws, *wr, *we, *gu, *grho;
     unsigned *wemax;
-    float cvs, crho, dh;
+    const float *cnorm;                   /* means of vs and rho */
+    float dh;
     int eprecond;
 };
+
+/* Means of vs and rho for the gradient normalisation, summed in the
+ * reference's order in float (x outer, depth inner; dsh_setup_cnorm): one
+ * thread per field adds in sequence from shared memory while the rest of the
+ * block fetches the next cb columns (or rc rows of one).  Bound by the chain of
+ * additions, 4 cycles each: 3.4 ms at 2000 x 800, beside the gradient's
+ * passes; on the host 2 ms of each dsh_set_model, needed or not. */
+__global__ void __launch_bounds__(256) cnorm_kernel(const float *vs, const float *rho, int nx, int ny, int pitch, int cb, int rc,
+                                                    float *out)
+{
+    extern __shared__ __align__(16) float sh[];
+    const int rp = (rc + 3) / 4 * 4, field = cb * rp, t = threadIdx.x;
+    const int nchunk = (ny + rc - 1) / rc, nblk = (nx + cb - 1) / cb * nchunk;
+    auto fetch = [&](int q) {
+        const int c0 = q / nchunk * cb, r0 = q % nchunk * rc, nc = min(cb, nx - c0), nr = min(rc, ny - r0);
+        float *d = sh + (q & 1) * 2 * field;
+        const long long o = (long long)r0 * pitch + HX + c0;
+#pragma unroll 4
+        for (int e = t - 64; e < nc * nr; e += 192) {
+            const int r = e / nc, c = e - r * nc;
+            const long long g = o + (long long)r * pitch + c;
+            d[c * rp + r] = __ldg(vs + g);
+            d[field + c * rp + r] = __ldg(rho + g);
+        }
+    };
+    if (t >= 64) fetch(0);
+    __syncthreads();
+    float s = 0.0f;
+    for (int q = 0; q < nblk; q++) {
+        if (t >= 64) {
+            if (q + 1 < nblk) fetch(q + 1);
+        } else if ((t & 31) == 0) {
+            const int c0 = q / nchunk * cb, r0 = q % nchunk * rc, nc = min(cb, nx - c0), nr = min(rc, ny - r0);
+            for (int c = 0; c < nc; c++) {
+                const float *d = sh + (q & 1) * 2 * field + (t >> 5) * field + c * rp;
+                int r = 0;
+#pragma unroll 4
+                for (; r + 4 <= nr; r += 4) {
+                    const float4 v = *reinterpret_cast<const float4 *>(d + r);
+                    s = s + v.x; s = s + v.y; s = s + v.z; s = s + v.w;
+                }
+                for (; r < nr; r++) s = s + d[r];
+            }
+        }
+        __syncthreads();
+    }
+    if (t == 0 || t == 32) out[t >> 5] = s / (float)((long long)nx * ny);
+}
 
 /* We = sqrt(Ws*Wr) (EPRECOND=1) or sqrt(Ws)*(asinh((xmax-x)/y)-asinh((xmin-x)/y))
  * (EPRECOND=3, Plessix & Mulder), and its maximum (eprecond1.c:17-57). */
@@ -217,14 +266,14 @@ __global__ void eprecond_scale_kernel(EpiArgs a)
     const long long so = (long long)s * a.slot_stride;
     const long long n = (long long)a.nx * a.ny;
     const float eps = 0.005f;
-    const float mx = __uint_as_float(a.wemax[s]);
+    const float mx = __uint_as_float(a.wemax[s]), cvs = __ldg(a.cnorm), crho = __ldg(a.cnorm + 1);
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(idx % a.nx) + 1, j = (int)(idx / a.nx) + 1;
         const long long o = so + (long long)(j - 1) * a.pitch + (i - 1 + HX);
         const float we = a.we[o] + (eps * mx);
         a.we[o] = we;
-        a.gu[o] = a.gu[o] / (we * a.cvs * a.cvs);
-        a.grho[o] = a.grho[o] / (we * a.crho * a.crho);
+        a.gu[o] = a.gu[o] / (we * cvs * cvs);
+        a.grho[o] = a.grho[o] / (we * crho * crho);
     }
 }
 
@@ -482,8 +531,11 @@ extern "C" dsh_ctx *dsh_create(const dsh_params *p, int device, int *status)
     if (cudaEventCreateWithFlags(&ctx->ev_wait, cudaEventDisableTiming) != cudaSuccess) return bail(DSH_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess)
+        cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&ctx->st_cnorm, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_cnorm, cudaEventDisableTiming) != cudaSuccess)
         return bail(DSH_ERR_CUDA);
+    if (cudaMalloc(&ctx->d_cnorm, 2 * sizeof(float)) != cudaSuccess) return bail(DSH_ERR_OOM);
     const int nx = p->nx, ny = p->ny, L = p->l, fw = p->fw;
     ctx->H = p->fdorder / 2;
     ctx->hy = ctx->H;
@@ -528,7 +580,7 @@ extern "C" dsh_ctx *dsh_create(const dsh_params *p, int device, int *status)
     ctx->slot_stride = o;
     if (cudaMalloc(&ctx->slab, (size_t)ctx->S * ctx->slot_stride * sizeof(float)) != cudaSuccess) return bail(DSH_ERR_OOM);
     build_tmaps(ctx);
-    const long long nmodel = 10LL * ctx->dstride;
+    const long long nmodel = (10LL + (p->grad_q ? 4 : 0)) * ctx->dstride;
     if (cudaMalloc(&ctx->model, (size_t)nmodel * sizeof(float)) != cudaSuccess) return bail(DSH_ERR_OOM);
     cudaMemset(ctx->model, 0, (size_t)nmodel * sizeof(float));
     float *m = ctx->model;
@@ -541,7 +593,8 @@ extern "C" dsh_ctx *dsh_create(const dsh_params *p, int device, int *status)
     ctx->m_taus = m; m += ctx->dstride;
     ctx->m_vs = m; m += ctx->dstride;
     ctx->m_rho = m; m += ctx->dstride;
-    ctx->m_qs = m;
+    ctx->m_qs = m; m += ctx->dstride;
+    ctx->m_qsens = m;                     /* 4 fields (grad_q) */
     if (cudaMalloc(&ctx->pml, 12 * (size_t)(2 * DSH_MAX_FW + 1) * sizeof(float)) != cudaSuccess) return bail(DSH_ERR_OOM);
     if (cudaMalloc(&ctx->sums, (p->grad_q ? 8 : 6) * (size_t)ctx->dstride * sizeof(float)) != cudaSuccess)
         return bail(DSH_ERR_OOM);
@@ -597,6 +650,9 @@ extern "C" int dsh_destroy(dsh_ctx *ctx)
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     if (ctx->st2) cudaStreamDestroy(ctx->st2);
+    if (ctx->ev_cnorm) cudaEventDestroy(ctx->ev_cnorm);
+    if (ctx->st_cnorm) { cudaStreamSynchronize(ctx->st_cnorm); cudaStreamDestroy(ctx->st_cnorm); }
+    cudaFree(ctx->d_cnorm);
     if (ctx->own_st) cudaStreamDestroy(ctx->own_st);
     delete ctx;
     return DSH_OK;
@@ -711,6 +767,25 @@ static __global__ void model_coef_kernel(ModelArgs m)
     }
 }
 
+/* Model factors of the forward pass's tau sensitivities (SF_QSENS in s_body):
+ * d(fipjp)/dtau = muip DT (L - sumu) / (1 + sumu tau) and
+ * (DT/2) / (tau (1 + sumu tau)) for both stresses, once per model instead of
+ * four divisions per point and step. */
+static __global__ void qsens_coef_kernel(int nx, int ny, int pitch, long long dstride, float dt, float dthalbe, float lf,
+                                         float sumu, const float *mi, const float *mj, const float *ti, const float *tj,
+                                         float *out)
+{
+    const long long n = (long long)nx * ny;
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const long long o = q / nx * pitch + q % nx + HX;
+        const float tx = ti[o], ty = tj[o], denx = 1.0f + sumu * tx, deny = 1.0f + sumu * ty;
+        out[o] = ((mi[o] * dt) * (lf - sumu)) / denx;
+        out[o + dstride] = ((mj[o] * dt) * (lf - sumu)) / deny;
+        out[o + 2 * dstride] = dthalbe / (tx * denx);
+        out[o + 3 * dstride] = dthalbe / (ty * deny);
+    }
+}
+
 static int upload_field(dsh_ctx *ctx, float *dst, const float *src)
 {
     CK(cudaMemcpy2DAsync(dst + HX, (size_t)ctx->pitch * sizeof(float), src, (size_t)ctx->p.nx * sizeof(float),
@@ -762,8 +837,12 @@ extern "C" int dsh_set_model(dsh_ctx *ctx, const float *vs, const float *rho, co
     ma.muip = ctx->m_muip; ma.mujp = ctx->m_mujp; ma.tip = ctx->m_tip; ma.taus = ctx->m_taus;
     model_coef_kernel<<<(unsigned)std::min<long long>(((long long)n + 255) / 256, 148LL * 8), 256, 0, ctx->st>>>(ma);
     CK(cudaGetLastError());
-    /* meanwhile on the host: the vs/rho means (a sequential float sum in the reference's order) */
-    dsh_setup_cnorm(p.nx, p.ny, vs, rho, ctx->cnorm);
+    if (p.grad_q)
+        qsens_coef_kernel<<<(unsigned)std::min<long long>(((long long)n + 255) / 256, 148LL * 8), 256, 0, ctx->st>>>(
+            p.nx, p.ny, ctx->pitch, ctx->dstride, p.dt, (float)((double)p.dt / 2.0), (float)L, ctx->sumu, ctx->m_muip,
+            ctx->m_mujp, ctx->m_tip, ctx->m_taus, ctx->m_qsens);
+    CK(cudaGetLastError());
+    ctx->cnorm_ok = 0;
     ctx->gq_valid = 0;
     WAIT(ctx);   /* the caller's arrays and the staging vector are free again once this returns */
     ctx->model_set = 1;
@@ -1123,6 +1202,7 @@ StepArgs step_args(dsh_ctx *ctx, Pass pass)
     a.lf = (float)p.l;
     a.sumu = ctx->sumu;
     if (p.grad_q) {
+        a.fipjp = ctx->m_qsens;
         a.exy = sl + ctx->o_exy; a.eyz = sl + ctx->o_eyz; a.gqx = sl + ctx->o_gqx; a.gqy = sl + ctx->o_gqy;
     }
     for (int l = 0; l < 4; l++) { a.bip[l] = ctx->bip[l]; a.bjm[l] = ctx->bjm[l]; a.cip[l] = ctx->cip[l]; a.cjm[l] = ctx->cjm[l]; }
@@ -1934,6 +2014,17 @@ static int gradient_impl(dsh_ctx *ctx, const dsh_shot *shots, int nshots, const 
     float ms_f = 0, ms_a = 0;
     long long out = 0;
     CK(cudaEventRecord(ctx->ev[0], ctx->st));
+    if ((p.eprecond == 1 || p.eprecond == 3) && !ctx->cnorm_ok) {   /* beside the passes; the scaling waits for it */
+        const int cb = std::max(1, std::min({8, p.nx, 10000 / (p.ny + 4)})), rc_ = std::min(p.ny, 10000);
+        const size_t smem = 4 * sizeof(float) * (size_t)cb * ((rc_ + 3) / 4 * 4);
+        CK(cudaFuncSetAttribute((const void *)cnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+        CK(cudaStreamWaitEvent(ctx->st_cnorm, ctx->ev[0], 0));
+        cnorm_kernel<<<1, 256, smem, ctx->st_cnorm>>>(ctx->m_vs, ctx->m_rho, p.nx, p.ny, ctx->pitch, cb, rc_, ctx->d_cnorm);
+        CK(cudaGetLastError());
+        CK(cudaEventRecord(ctx->ev_cnorm, ctx->st_cnorm));
+        ctx->launches++;
+        ctx->cnorm_ok = 1;
+    }
     for (int b0 = 0; b0 < nshots; b0 += ctx->S) {
         const int nb = std::min(ctx->S, nshots - b0);
         const float *obs_h = obs_host ? obs_host + out : nullptr;
@@ -1989,7 +2080,8 @@ static int gradient_impl(dsh_ctx *ctx, const dsh_shot *shots, int nshots, const 
             ea.nx = p.nx; ea.ny = p.ny; ea.pitch = ctx->pitch; ea.slot_stride = ctx->slot_stride;
             ea.ws = ctx->slab + ctx->o_ws; ea.wr = ctx->slab + ctx->o_wr; ea.we = ctx->slab + ctx->o_we;
             ea.gu = ctx->slab + ctx->o_gu; ea.grho = ctx->slab + ctx->o_grho;
-            ea.wemax = ctx->d_wemax; ea.cvs = ctx->cnorm[0]; ea.crho = ctx->cnorm[1]; ea.dh = p.dh;
+            ea.wemax = ctx->d_wemax; ea.cnorm = ctx->d_cnorm; ea.dh = p.dh;
+            CK(cudaStreamWaitEvent(ctx->st, ctx->ev_cnorm, 0));
             ea.eprecond = p.eprecond;
             CK(cudaMemsetAsync(ctx->d_wemax, 0, (size_t)nb * sizeof(unsigned), ctx->st));
             eprecond_we_kernel<<<epi_grid(ctx, nb), 256, 0, ctx->st>>>(ea);

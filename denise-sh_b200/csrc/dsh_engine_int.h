@@ -47,9 +47,14 @@ struct dsh_ctx {
     float eta[4] = {0};
     float *pml = nullptr;
     float *sums = nullptr;                /* sum_u, sum_rho, out_a, out_b (dense pitched) */
-    float hc[7] = {0}, bip[4] = {0}, bjm[4] = {0}, cip[4] = {0}, cjm[4] = {0}, cnorm[2] = {0};
+    float hc[7] = {0}, bip[4] = {0}, bjm[4] = {0}, cip[4] = {0}, cjm[4] = {0};
     int pml_k1 = 0;                       /* every CPML stretching K is 1 */
     float rdh_h = 0.0f, rdh_l = 0.0f, rdh_lo = INFINITY;   /* div_dh's product form (StepArgs) */
+    float *d_cnorm = nullptr;             /* means of vs and rho (cnorm_kernel), formed by the first gradient of a model */
+    int cnorm_ok = 0;
+    cudaStream_t st_cnorm = nullptr;
+    cudaEvent_t ev_cnorm = nullptr;
+    float *m_qsens = nullptr;             /* factors of the tau sensitivities (grad_q) */
     int model_set = 0;
     float *fwd = nullptr;
     long long fwd_slot_stride = 0, fwd_step_stride = 0;

@@ -121,7 +121,9 @@ struct StepArgs {
     float *vy, *sxy, *syz, *r, *q, *psi_vxx, *psi_vyy_v, *psi_sxx, *psi_syy;
     float *ws, *gu, *grho, *hu, *hrho;
     /* model (shared by all slots) */
-    const float *brho, *uip, *ujp, *fipjp, *f, *dip, *d;
+    const float *brho, *uip, *ujp;
+    const float *fipjp;          /* SF_PARAMS; with SF_QSENS the four fields ax, ay, kx, ky of the sensitivities */
+    const float *f, *dip, *d;
     const float *muip, *mujp, *tausipjp, *taus;   /* viscoelastic base factors */
     float eta[4];                /* DT / tau_l */
     float lf;                    /* L as a float */
@@ -1234,16 +1236,15 @@ __device__ __forceinline__ void s_body(const StepArgs &a, int nt_off, int i0, in
             /* d(stress increment)/d(tau) with the strain history held fixed:
                dfipjp/dtau = muip DT (L - sumu) / (1 + sumu tau), and every memory
                variable scales with its dip_l, whose log-derivative is
-               1 / (tau (1 + sumu tau)) (prepare_update_s.c:40-55) */
+               1 / (tau (1 + sumu tau)) (prepare_update_s.c:40-55); the factors
+               come from the model (qsens_coef_kernel) */
+            const float *qc = a.fipjp + drow + col0;
+            const float4 ax = ldg4p(qc, pol_f), ay = ldg4p(qc + a.dstride, pol_f);
+            const float4 kx = ldg4p(qc + 2 * a.dstride, pol_f), ky = ldg4p(qc + 3 * a.dstride, pol_f);
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                const float tx = get(ti4, k), ty = get(tj4, k);
-                const float denx = 1.0f + a.sumu * tx, deny = 1.0f + a.sumu * ty;
-                const float ax = ((get(mi4, k) * a.dt) * (a.lf - a.sumu)) / denx;
-                const float ay = ((get(mj4, k) * a.dt) * (a.lf - a.sumu)) / deny;
-                const float kx = a.dthalbe / (tx * denx), ky = a.dthalbe / (ty * deny);
-                set(qsx, k, (ax * get(vyx4, k)) + (kx * (get(sold_r, k) + get(sumr4, k))));
-                set(qsy, k, (ay * get(vyy4, k)) + (ky * (get(sold_q, k) + get(sumq4, k))));
+                set(qsx, k, (get(ax, k) * get(vyx4, k)) + (get(kx, k) * (get(sold_r, k) + get(sumr4, k))));
+                set(qsy, k, (get(ay, k) * get(vyy4, k)) + (get(ky, k) * (get(sold_q, k) + get(sumq4, k))));
             }
         }
     }

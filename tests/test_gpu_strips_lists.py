@@ -17,6 +17,7 @@ CASES = [  # nx, ny, fw, fdorder, L, free_surf, dh, k_max, nrow
     (61, 33, 10, 10, 0, 1, 1.1, 1.5, 33),
     (141, 21, 6, 4, 3, 0, 0.7, 2.0, 70),
     (262, 19, 5, 8, 0, 1, 0.5, 3.0, 131),
+    (21, 10050, 4, 2, 0, 1, 0.5, 1.0, 9),   # more rows than one block of the vs / rho means holds
 ]
 
 
