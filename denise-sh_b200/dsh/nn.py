@@ -1,8 +1,8 @@
 """Learned pseudo-Hessian preconditioner: a 4-level U-Net whose every
 convolution, pooling, activation, loss and optimiser step runs in the
 in-tree CUDA library ``libdsh_nn.so`` (include/dsh_nn.h): 3x3 convolutions
-are im2col + a tcgen05/TMA BF16 GEMM with FP32 accumulation in tensor
-memory.  PyTorch only provides device memory and the stream.
+are implicit tcgen05/TMA BF16 GEMMs with FP32 accumulation in tensor memory
+(the first layer and the weight gradients through column matrices).  PyTorch only provides device memory and the stream.
 
 Network (NHWC, H and W divisible by 8):
     enc1 conv(8->32) conv(32->32) | pool | enc2 conv(32->64) conv(64->64) | pool
@@ -40,6 +40,7 @@ def nnlib() -> C.CDLL:
         v, i, ll, f = C.c_void_p, C.c_int, C.c_longlong, C.c_float
         L.dsh_nn_gemm.argtypes = [i, i, i, v, ll, v, ll, v, v, ll, v, i, i, v, i, v, v]
         L.dsh_nn_set_wait_limit.argtypes = [ll]
+        L.dsh_nn_conv3x3.argtypes = [v, i, i, i, i, v, ll, i, v, v, v, i, v, v]
         L.dsh_nn_im2col.argtypes = [v, i, i, i, i, v, ll, v]
         L.dsh_nn_im2col_t.argtypes = [v, i, i, i, i, v, ll, v]
         L.dsh_nn_transpose.argtypes = [v, ll, i, v, ll, v]
@@ -116,6 +117,10 @@ class Ctx:
         _ck(nnlib().dsh_nn_gemm(M, N, K, _p(A), lda, _p(B), ldb, _p(c32), _p(c16), ldc, _p(bias), int(relu),
                                 splits, _p(part), int(accumulate), _p(self.err), self.st), "dsh_nn_gemm")
 
+    def conv3x3(self, x, B, H, W, C, w, ldw, N, c32=None, c16=None, bias=None, relu=False):
+        _ck(nnlib().dsh_nn_conv3x3(_p(x), B, H, W, C, _p(w), ldw, N, _p(c32), _p(c16), _p(bias), int(relu), _p(self.err),
+                                   self.st), "dsh_nn_conv3x3")
+
     def check(self):
         self.torch.cuda.synchronize()
         e = int(self.err.item())
@@ -152,6 +157,9 @@ class Conv3x3:
         """x bf16 [P][cin] -> y bf16 [P][cout] (ReLU applied)."""
         ctx = self.ctx
         P = B * H * W
+        if self.cin % 32 == 0:
+            ctx.conv3x3(x, B, H, W, self.cin, self.wb, self.ldk, self.cout, c16=y, bias=self.b, relu=True)
+            return
         col = ctx.scratch("col", P * self.ldk, ctx.torch.bfloat16)
         _ck(nnlib().dsh_nn_im2col(_p(x), B, H, W, self.cin, _p(col), self.ldk, ctx.st), "im2col")
         ctx.gemm(P, self.cout, self.K, col, self.ldk, self.wb, self.ldk, c16=y, bias=self.b, relu=True)
@@ -173,7 +181,9 @@ class Conv3x3:
         _ck(nnlib().dsh_nn_transpose(_p(dz), P, self.cout, _p(dzT), ldp, ctx.st), "transpose")
         splits = max(1, min(64, P // 8192))
         ctx.gemm(self.K, self.cout, P, colT, ldp, dzT, ldp, c32=self.gwt, splits=splits, accumulate=True)
-        if dx is not None:
+        if dx is not None and self.cout % 32 == 0:
+            ctx.conv3x3(dz, B, H, W, self.cout, self.wf, self.ldf, self.cin, c32=dx)
+        elif dx is not None:
             col = ctx.scratch("col", P * self.ldf, torch.bfloat16)
             _ck(nnlib().dsh_nn_im2col(_p(dz), B, H, W, self.cout, _p(col), self.ldf, ctx.st), "im2col")
             ctx.gemm(P, self.cin, 9 * self.cout, col, self.ldf, self.wf, self.ldf, c32=dx)

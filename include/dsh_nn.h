@@ -46,6 +46,14 @@ int dsh_nn_gemm(int M, int N, int K, const void *A, long long lda, const void *B
                 long long ldc, const float *bias, int relu, int splits, float *partial, int accumulate, int *err,
                 void *stream);
 
+/* 3x3 same-padded convolution on the tensor cores without a column matrix:
+ * x bf16 [B][H][W][C], w bf16 [N][ldw] with columns tap*C + c, result [P][N]
+ * as float (C32) and/or bf16 (C16), bias and ReLU as dsh_nn_gemm; the same
+ * bits as dsh_nn_im2col + dsh_nn_gemm.  C a multiple of 32, N and ldw of 8,
+ * 16-byte aligned bases. */
+int dsh_nn_conv3x3(const void *x, int B, int H, int W, int C, const void *w, long long ldw, int N, float *C32, void *C16,
+                   const float *bias, int relu, int *err, void *stream);
+
 /* im2col of a 3x3 same-padded convolution: x bf16 [B][H][W][C] ->
  * col bf16 [P][ldk] (columns 9C..ldk-1 are left untouched) */
 int dsh_nn_im2col(const void *x, int B, int H, int W, int C, void *col, long long ldk, void *stream);

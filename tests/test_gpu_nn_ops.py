@@ -118,3 +118,29 @@ def test_relu_backward_add_and_column_sums(P, N, off):
     assert L.dsh_nn_add(dy.data_ptr(), other.data_ptr(), P * N, None) == 0
     torch.cuda.synchronize()
     assert torch.equal(dy, s)
+
+
+@pytest.mark.parametrize("B,H,W,C,N", [(1, 1, 1, 32, 32), (2, 9, 17, 32, 64), (1, 8, 16, 64, 8), (1, 25, 75, 96, 32),
+                                       (1, 13, 40, 128, 256), (2, 7, 15, 256, 128), (1, 16, 33, 64, 288)])
+def test_convolution_equals_columns_and_gemm(B, H, W, C, N):
+    """The implicit convolution gives the bits of im2col + GEMM, with and without bias and ReLU, at tiles of 8 x 16 pixels
+    with remainders, both K block sizes and every N tile."""
+    torch, L = _env()
+    from dsh import nn as dnn
+
+    P, K = B * H * W, 9 * C
+    ctx = dnn.Ctx(torch)
+    x = torch.randn(P * C, device="cuda").bfloat16()
+    w = (torch.randn(N * K, device="cuda") / K ** 0.5).bfloat16()
+    bias = torch.randn(N, device="cuda")
+    col = torch.empty(P * K, dtype=torch.bfloat16, device="cuda")
+    assert L.dsh_nn_im2col(x.data_ptr(), B, H, W, C, col.data_ptr(), K, None) == 0
+    for b, relu in ((None, False), (bias, True)):
+        want16, got16 = torch.empty(P * N, dtype=torch.bfloat16, device="cuda"), _buf(torch, P * N, torch.bfloat16)
+        ctx.gemm(P, N, K, col, K, w, K, c16=want16, bias=b, relu=relu)
+        ctx.conv3x3(x, B, H, W, C, w, K, N, c16=got16, bias=b, relu=relu)
+        want32, got32 = torch.empty(P * N, device="cuda"), _buf(torch, P * N, torch.float32)
+        ctx.gemm(P, N, K, col, K, w, K, c32=want32, bias=b, relu=relu)
+        ctx.conv3x3(x, B, H, W, C, w, K, N, c32=got32, bias=b, relu=relu)
+        ctx.check()
+        assert torch.equal(got16, want16) and torch.equal(got32, want32)
