@@ -86,42 +86,59 @@ __global__ void im2col_v8(const uint4 *x, int H, int W, unsigned nc, unsigned n,
     col[(long long)p * ldk8 + k] = v;
 }
 
-/* Transposed columns (TAPS 9) or a plain transpose (TAPS 1) of a tile of 64
- * pixels x 32 channels through shared memory: 16-byte loads along the
- * channels, 16-byte stores along the pixels.  Pitch 66: the 2-byte stores of a
- * warp (8 pixels x 4 vectors of 8 channels) fall into different banks.  The
- * 17 launches of a training step on two 400 x 1200 maps: 22.5 ms with the
- * one-element kernel, 2.6 ms with this one. */
+/* Transposed columns (TAPS 9) or a plain transpose (TAPS 1) of a tile of 128
+ * pixels x 32 channels through shared memory: a thread loads 8 channels of
+ * two neighbouring pixels (16 bytes each), stores eight pixel pairs, and
+ * writes 16 bytes along the pixels.  Pitch 65 words: the stores of a warp (8
+ * pairs x 4 vectors of 8 channels) fall into different banks.  The 17 launches
+ * of a training step on two 400 x 1200 maps: 22.5 ms with the one-element
+ * kernel, 2.6 ms one pixel per thread, 2.3 ms with this one (6.3 GB written). */
 template <int TAPS>
 __global__ void __launch_bounds__(256) transpose_v8(const uint4 *x, int H, int W, int C, int P, bf16 *yT, long long ldp)
 {
-    __shared__ __align__(16) uint16_t t[32][66];
+    __shared__ uint32_t t[32 * 65];
     const int tap = TAPS == 9 ? blockIdx.z : 4;
-    const int p0 = blockIdx.x * 64, c0 = blockIdx.y * 32;
+    const int p0 = blockIdx.x * 128, c0 = blockIdx.y * 32;
     {
-        const int r = threadIdx.x >> 2, v8 = threadIdx.x & 3, p = p0 + r, c = c0 + 8 * v8;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        bool in = p < P && c < C;
-        long long q = p;
-        if (TAPS == 9 && in) {
-            const int row = p / W, xx = p - row * W + tap % 3 - 1, yy = row % H + tap / 3 - 1;
-            in = yy >= 0 && yy < H && xx >= 0 && xx < W;
-            q += (tap / 3 - 1) * W + tap % 3 - 1;
-        }
-        if (in) v = __ldg(x + (q * C + c) / 8);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        const int pair = threadIdx.x >> 2, v8 = threadIdx.x & 3, c = c0 + 8 * v8;
+        uint4 v[2];
 #pragma unroll
-        for (int e = 0; e < 8; e++) t[8 * v8 + e][r] = (uint16_t)(w[e >> 1] >> (16 * (e & 1)));
+        for (int h = 0; h < 2; h++) {
+            const int p = p0 + 2 * pair + h;
+            v[h] = make_uint4(0, 0, 0, 0);
+            bool in = p < P && c < C;
+            long long q = p;
+            if (TAPS == 9 && in) {
+                const int row = p / W, xx = p - row * W + tap % 3 - 1, yy = row % H + tap / 3 - 1;
+                in = yy >= 0 && yy < H && xx >= 0 && xx < W;
+                q += (tap / 3 - 1) * W + tap % 3 - 1;
+            }
+            if (in) v[h] = __ldg(x + (q * C + c) / 8);
+        }
+        const uint32_t a[4] = {v[0].x, v[0].y, v[0].z, v[0].w}, b[4] = {v[1].x, v[1].y, v[1].z, v[1].w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            t[(8 * v8 + 2 * e) * 65 + pair] = __byte_perm(a[e], b[e], 0x5410);
+            t[(8 * v8 + 2 * e + 1) * 65 + pair] = __byte_perm(a[e], b[e], 0x7632);
+        }
     }
     __syncthreads();
-    const int cl = threadIdx.x >> 3, pv = threadIdx.x & 7, c = c0 + cl, p = p0 + 8 * pv;
-    if (c >= C || p >= P) return;
-    bf16 *dst = yT + ((TAPS == 9 ? (long long)tap * C : 0) + c) * ldp + p;
-    const uint32_t *src = reinterpret_cast<const uint32_t *>(&t[cl][8 * pv]);
-    if (p + 8 <= P)
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(src[0], src[1], src[2], src[3]);
-    else
-        for (int e = 0; p + e < P; e++) reinterpret_cast<uint16_t *>(dst)[e] = t[cl][8 * pv + e];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int k = threadIdx.x + 256 * h, cl = k >> 4, pv = k & 15, c = c0 + cl, p = p0 + 8 * pv;
+        if (c >= C || p >= P) continue;
+        bf16 *dst = yT + ((TAPS == 9 ? (long long)tap * C : 0) + c) * ldp + p;
+        const uint32_t *src = t + cl * 65 + 4 * pv;
+        const uint4 w = make_uint4(src[0], src[1], src[2], src[3]);
+        if (p + 8 <= P) {
+            *reinterpret_cast<uint4 *>(dst) = w;
+        } else {
+            const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                if (p + e < P) reinterpret_cast<uint16_t *>(dst)[e] = (uint16_t)(u[e >> 1] >> (16 * (e & 1)));
+        }
+    }
 }
 
 /* 32 x 32 tile transpose through shared memory */
@@ -370,6 +387,24 @@ __global__ void split_k(const float *dy, int C1, int C2, long long P, float *da,
     }
 }
 
+/* one thread per pixel, 16-byte loads, products added in channel order as above (C a multiple of 8) */
+__global__ void head_fwd_v8(const uint4 *x, unsigned P, int nc, const float *w, const float *b, float *out)
+{
+    VEC_INDEX(p, P);
+    float s = 0.0f;
+    for (int c = 0; c < nc; c++) {
+        const uint4 v = __ldg(x + (long long)p * nc + c);
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const float2 f = bf2(u[e]);
+            s += f.x * __ldg(w + 8 * c + 2 * e);
+            s += f.y * __ldg(w + 8 * c + 2 * e + 1);
+        }
+    }
+    out[p] = s + b[0];
+}
+
 __global__ void head_fwd_k(const bf16 *x, long long P, int C, const float *w, const float *b, float *out)
 {
     GRID_LOOP(p, P)
@@ -389,15 +424,29 @@ __global__ void head_bwd_k(const float *dout, const bf16 *x, long long P, int C,
 {
     const long long rows = (P + gridDim.x - 1) / gridDim.x;
     const long long r0 = (long long)blockIdx.x * rows, r1 = min(P, r0 + rows);
-    for (long long idx = r0 * C + threadIdx.x; idx < r1 * C; idx += blockDim.x) {
-        const long long p = idx / C;
-        dx[idx] = dout[p] * w[idx % C];
+    if (C % 4 == 0 && (((uintptr_t)dx | (uintptr_t)w) & 15) == 0) {
+        const unsigned nv = C / 4, n = (unsigned)max(r1 - r0, 0LL) * nv;
+        float4 *o = reinterpret_cast<float4 *>(dx + r0 * C);
+        const float4 *wv = reinterpret_cast<const float4 *>(w);
+#pragma unroll 4
+        for (unsigned i = threadIdx.x; i < n; i += blockDim.x) {
+            const unsigned p = i / nv;
+            const float d = __ldg(dout + r0 + p);
+            const float4 v = __ldg(wv + (i - p * nv));
+            o[i] = make_float4(d * v.x, d * v.y, d * v.z, d * v.w);
+        }
+    } else {
+        for (long long idx = r0 * C + threadIdx.x; idx < r1 * C; idx += blockDim.x) {
+            const long long p = idx / C;
+            dx[idx] = dout[p] * w[idx % C];
+        }
     }
     extern __shared__ float acc[];                 /* blockDim.x */
     const int W = C + 1, lanes = blockDim.x / W;
     float s = 0.0f;
     if ((int)threadIdx.x < lanes * W) {
         const int c = threadIdx.x % W, lane = threadIdx.x / W;
+#pragma unroll 8
         for (long long p = r0 + lane; p < r1; p += lanes)
             s += c < C ? dout[p] * __bfloat162float(x[p * C + c]) : dout[p];
     }
@@ -470,8 +519,13 @@ __global__ void sum_parts_k(const float *part, int nblocks, int N, int stride, f
 {
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
         float s = 0.0f;
-#pragma unroll 16
-        for (int b = 0; b < nblocks; b++) s += part[(long long)b * stride + n];
+        for (int b = 0; b < nblocks; b += 37) {          /* DSH_NN_RED_BLOCKS = 8 x 37: 37 loads in flight */
+            float v[37];
+#pragma unroll
+            for (int k = 0; k < 37; k++) v[k] = part[(long long)(b + k) * stride + n];
+#pragma unroll
+            for (int k = 0; k < 37; k++) s += v[k];
+        }
         g[n] += s;
     }
 }
@@ -533,7 +587,7 @@ extern "C" int dsh_nn_im2col_t(const void *x, int B, int H, int W, int C, void *
     if (!x || !colT || B <= 0 || H <= 0 || W <= 0 || C <= 0 || ldp < (long long)B * H * W) return DSH_NN_ERR_PARAM;
     const long long n = (long long)B * H * W * 9 * C, P = (long long)B * H * W;
     if (vec_ok(P, C) && ldp % 8 == 0 && al16(x) && al16(colT) && C <= 32 * 65535) {
-        transpose_v8<9><<<dim3((unsigned)((P + 63) / 64), (unsigned)((C + 31) / 32), 9), 256, 0, ST>>>(
+        transpose_v8<9><<<dim3((unsigned)((P + 127) / 128), (unsigned)((C + 31) / 32), 9), 256, 0, ST>>>(
             (const uint4 *)x, H, W, C, (int)P, (bf16 *)colT, ldp);
         return status();
     }
@@ -545,7 +599,7 @@ extern "C" int dsh_nn_transpose(const void *y, long long P, int C, void *yT, lon
 {
     if (!y || !yT || P <= 0 || C <= 0 || ldp < P) return DSH_NN_ERR_PARAM;
     if (vec_ok(P, C) && ldp % 8 == 0 && al16(y) && al16(yT) && C <= 32 * 65535) {
-        transpose_v8<1><<<dim3((unsigned)((P + 63) / 64), (unsigned)((C + 31) / 32), 1), 256, 0, ST>>>(
+        transpose_v8<1><<<dim3((unsigned)((P + 127) / 128), (unsigned)((C + 31) / 32), 1), 256, 0, ST>>>(
             (const uint4 *)y, 1, 1, C, (int)P, (bf16 *)yT, ldp);
         return status();
     }
@@ -670,11 +724,16 @@ extern "C" int dsh_nn_head_fwd(const void *x, long long P, int C, const float *w
                                void *stream)
 {
     if (!x || !w || !b || !out || P <= 0 || C <= 0) return DSH_NN_ERR_PARAM;
+    if (vec_ok(P, C) && al16(x)) {
+        head_fwd_v8<<<vgrid(P), 256, 0, ST>>>((const uint4 *)x, (unsigned)P, C / 8, w, b, out);
+        return status();
+    }
     head_fwd_k<<<grid_for(P), 256, 0, ST>>>((const bf16 *)x, P, C, w, b, out);
     return status();
 }
 
 constexpr int RED_BLOCKS = DSH_NN_RED_BLOCKS;
+static_assert(RED_BLOCKS % 37 == 0, "sum_parts_k");
 
 extern "C" int dsh_nn_head_bwd(const float *dout, const void *x, long long P, int C, const float *w, float *dx,
                                float *gw, float *gb, float *part, void *stream)
