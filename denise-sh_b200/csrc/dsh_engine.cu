@@ -1641,12 +1641,14 @@ static bool tblock_cfg(dsh_ctx *ctx, Pass pass, int nb, TbProblem *pb, TbCfg *cf
     pb->max_entries = pass == P_ADJ ? ctx->geo_max_ntr : ctx->geo_max_src;
     pb->max_members = pass == P_ADJ ? ctx->geo_max_adj_members : ctx->geo_max_members;
     pb->max_receivers = pass == P_ADJ ? 0 : ctx->geo_max_ntr;
-    /* unless asked for, only with two steps or more between two exchanges (us
-       per step against the pair's: 160 x 80, FDORDER 4, k 4: 2.2 and 4.1; 500 x
-       200: 2.9 and 4.6; 700 x 280: 3.6 and 5.1; FDORDER 8, k 2: 3.5 and 4.3, 4.3
-       and 4.9; with one step the pair is faster: 1000 x 300 6.8 and 5.4, 700 x
-       280, FDORDER 8: 7.0 and 6.0) */
-    pb->min_k = ctx->sel_tblock > 0 || env ? 1 : 2;
+    /* unless asked for, only with two steps or more between two exchanges and
+       up to 262144 points (us per step against the pair's: 160 x 80, FDORDER 4, k
+       4: 1.9 and 4.0; 500 x 200: 2.5 and 4.4; 700 x 280: 3.6 and 4.7; FDORDER 8, k 2:
+       3.5 and 4.0, 4.4 and 4.7; 3 shots of 500 x 200 5.3 and 5.1; with one step 1000
+       x 300 7.1 and 4.9, 700 x 280, FDORDER 8: 7.2 and 5.5) */
+    const bool asked = ctx->sel_tblock > 0 || env;
+    if (!asked && (long long)p.nx * p.ny * nb > 1 << 18) return false;
+    pb->min_k = asked ? 1 : 2;
     return tb_config(*pb, cfg);
 }
 

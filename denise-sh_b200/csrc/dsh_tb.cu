@@ -27,11 +27,16 @@ static TbFn tb_pick(int fdo, int mode)
     }
 }
 
+template <int MAXT>
+static TbFn tb_p2(const TbProblem &pb)
+{
+    return pb.p2 ? tb_pick<true, MAXT>(pb.fdorder, pb.mode) : tb_pick<false, MAXT>(pb.fdorder, pb.mode);
+}
 static TbFn tb_fn(const TbProblem &pb, int nthr)
 {
-    if (nthr <= TB_FEW_THREADS)
-        return pb.p2 ? tb_pick<true, TB_FEW_THREADS>(pb.fdorder, pb.mode) : tb_pick<false, TB_FEW_THREADS>(pb.fdorder, pb.mode);
-    return pb.p2 ? tb_pick<true, TB_MAX_THREADS>(pb.fdorder, pb.mode) : tb_pick<false, TB_MAX_THREADS>(pb.fdorder, pb.mode);
+    return nthr <= TB_FEW_THREADS   ? tb_p2<TB_FEW_THREADS>(pb)
+           : nthr <= TB_MID_THREADS ? tb_p2<TB_MID_THREADS>(pb)
+                                    : tb_p2<TB_MAX_THREADS>(pb);
 }
 
 static int env_int(const char *name, int lo, int hi)
@@ -71,8 +76,12 @@ bool tb_config(const TbProblem &pb, TbCfg *cfg)
         const long long tiles = (long long)g.ntx * g.nty * pb.nb;
         const long long bytes = 4LL * tb_smem(g, H, pb.mode).total;
         if (g.nthr > TB_MAX_THREADS || tiles > nsm || bytes > maxsm) return false;
-        /* per step one vector of a thread, per round the exchange (us; 160 x 80: 1.3 + 2.8 / k, 500 x 200: 2.1 + 2.8 / k) */
-        const double step = 0.7 + 0.0021 * g.nthr, t = step + 2.8 / k;
+        /* per step one vector of a thread, slower with the fewer registers of
+           larger blocks, per round the exchange (us; 160 x 80, 448 threads: 1.2 +
+           2.8 / k, 500 x 200, 672 threads: 1.9 + 2.8 / k; one build with 64
+           registers: 1.5 and 2.1) */
+        const double few = g.nthr <= TB_FEW_THREADS ? 1.0 : g.nthr <= TB_MID_THREADS ? 1.05 : 1.2;
+        const double step = 0.5 + 0.0018 * g.nthr * few, t = step + 2.8 / k;
         if (best == 0.0 || t < best) {
             best = t;
             c.geo = g;

@@ -48,8 +48,8 @@
 
 namespace dsh {
 
-constexpr int TB_MAX_THREADS = 1024;     /* 64 registers per thread; blocks of up to TB_FEW_THREADS run the build with 96 */
-constexpr int TB_FEW_THREADS = 640;
+/* block sizes of the builds: 64, 88 and 128 registers per thread */
+constexpr int TB_MAX_THREADS = 1024, TB_MID_THREADS = 704, TB_FEW_THREADS = 512;
 constexpr int TB_MAX_ENT = 1024; /* sources of a slot (receivers in the adjoint) */
 constexpr int TB_MAX_MEM = 8;    /* sources at one point */
 constexpr int TB_MAX_REC = 2048; /* receivers of a slot */
