@@ -529,12 +529,6 @@ extern "C" dsh_ctx *dsh_create(const dsh_params *p, int device, int *status)
     ctx->st = ctx->own_st;
     for (int k = 0; k < 4; k++) cudaEventCreate(&ctx->ev[k]);
     if (cudaEventCreateWithFlags(&ctx->ev_wait, cudaEventDisableTiming) != cudaSuccess) return bail(DSH_ERR_CUDA);
-    if (cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&ctx->st_cnorm, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->ev_cnorm, cudaEventDisableTiming) != cudaSuccess)
-        return bail(DSH_ERR_CUDA);
     if (cudaMalloc(&ctx->d_cnorm, 2 * sizeof(float)) != cudaSuccess) return bail(DSH_ERR_OOM);
     const int nx = p->nx, ny = p->ny, L = p->l, fw = p->fw;
     ctx->H = p->fdorder / 2;
@@ -1435,6 +1429,16 @@ static int slot_split(const dsh_ctx *ctx, const VPick &vp, int nb)
     return on ? nb / 2 : 0;
 }
 
+/* the side stream of slot_split and of cnorm_kernel, and their events, when first needed (never during a capture) */
+static int side_stream(cudaStream_t *st, cudaEvent_t *e0, cudaEvent_t *e1, dsh_ctx *ctx)
+{
+    if (*st) return DSH_OK;
+    if (e0 && !*e0) CK(cudaEventCreateWithFlags(e0, cudaEventDisableTiming));
+    if (e1 && !*e1) CK(cudaEventCreateWithFlags(e1, cudaEventDisableTiming));
+    CK(cudaStreamCreateWithFlags(st, cudaStreamNonBlocking));
+    return DSH_OK;
+}
+
 static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chunk, long long *nlaunch, int slot0 = 0)
 {
     if (use_fused(ctx, pass)) return launch_fused_chunk(ctx, pass, nb, nsteps_in_chunk, nlaunch);
@@ -1667,12 +1671,11 @@ static int ensure_flags(dsh_ctx *ctx, long long n)
     return DSH_OK;
 }
 
-static int run_tblock(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, const TbProblem &pb, const TbCfg &cfg)
+/* flags and exchange planes of the blocked pass; without room for them the
+ * kernel pair serves the pass */
+static bool tblock_buffers(dsh_ctx *ctx, int nb, const TbCfg &cfg)
 {
-    StepArgs sa = step_args(ctx, pass);
-    sa.nslots = nb;
-    int rc = ensure_flags(ctx, cfg.tiles);
-    if (rc != DSH_OK) return rc;
+    if (ensure_flags(ctx, cfg.tiles) != DSH_OK) return false;
     const long long need = 2LL * nb * TB_XFIELDS * ctx->dstride;
     if (need > ctx->tb_cap) {
         cudaFree(ctx->d_tb);
@@ -1680,10 +1683,17 @@ static int run_tblock(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, const 
         ctx->tb_cap = 0;
         if (cudaMalloc(&ctx->d_tb, (size_t)need * sizeof(float)) != cudaSuccess) {
             cudaGetLastError();
-            return DSH_ERR_OOM;
+            return false;
         }
         ctx->tb_cap = need;
     }
+    return true;
+}
+
+static int run_tblock(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, const TbProblem &pb, const TbCfg &cfg)
+{
+    StepArgs sa = step_args(ctx, pass);
+    sa.nslots = nb;
     CK(cudaMemsetAsync(ctx->d_flags, 0, (size_t)cfg.tiles * sizeof(unsigned), ctx->st));
     CK(tb_launch(cfg, pb, sa, TbExchange{ctx->d_tb, ctx->d_flags}, n0, count, ctx->st));
     ctx->launches += 1;
@@ -1744,8 +1754,10 @@ static int run_steps(dsh_ctx *ctx, Pass pass, int nb, int n0, int count)
     if (cluster_cfg(ctx, pass, nb, &ccfg)) return run_cluster(ctx, pass, nb, n0, count, ccfg);
     TbCfg tcfg;
     TbProblem tpb;
-    if (tblock_cfg(ctx, pass, nb, &tpb, &tcfg)) return run_tblock(ctx, pass, nb, n0, count, tpb, tcfg);
+    if (tblock_cfg(ctx, pass, nb, &tpb, &tcfg) && tblock_buffers(ctx, nb, tcfg)) return run_tblock(ctx, pass, nb, n0, count, tpb, tcfg);
     if (const int grid = persistent_grid(ctx, pass, nb)) return run_persistent(ctx, pass, nb, n0, count, grid);
+    const int rc_side = nb > 1 ? side_stream(&ctx->st2, &ctx->ev_fork, &ctx->ev_join, ctx) : DSH_OK;
+    if (rc_side != DSH_OK) return rc_side;
     if (const int group = slot_group(ctx, pass, nb)) return run_groups(ctx, pass, nb, n0, count, group);
     const int K = std::min(ctx->chunk, count);
     const int nfull = count / K, rem = count % K;
@@ -2020,6 +2032,7 @@ static int gradient_impl(dsh_ctx *ctx, const dsh_shot *shots, int nshots, const 
         const int cb = std::max(1, std::min({8, p.nx, 10000 / (p.ny + 4)})), rc_ = std::min(p.ny, 10000);
         const size_t smem = 4 * sizeof(float) * (size_t)cb * ((rc_ + 3) / 4 * 4);
         CK(cudaFuncSetAttribute((const void *)cnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+        if ((rc = side_stream(&ctx->st_cnorm, &ctx->ev_cnorm, nullptr, ctx)) != DSH_OK) return rc;
         CK(cudaStreamWaitEvent(ctx->st_cnorm, ctx->ev[0], 0));
         cnorm_kernel<<<1, 256, smem, ctx->st_cnorm>>>(ctx->m_vs, ctx->m_rho, p.nx, p.ny, ctx->pitch, cb, rc_, ctx->d_cnorm);
         CK(cudaGetLastError());

@@ -1,42 +1,20 @@
-/* Instantiations, launch shape and launch of the temporally blocked pass of
- * small elastic grids (dsh_tblock.cuh), FDORDER 2..8. */
+/* Launch shape and launch of the temporally blocked pass of small elastic
+ * grids (dsh_tblock.cuh), FDORDER 2..8. */
 #include <algorithm>
 #include <cstdlib>
 
 #include "dsh_tb.h"
 
 namespace dsh {
-using TbFn = void (*)(StepArgs, TbGeom, TbExchange, int, int);
-
-template <int FDO, bool P2, int MAXT>
-static TbFn tb_mode(int mode)
-{
-    return mode == TB_ADJ     ? tb_pass<FDO, P2, TB_ADJ, MAXT>
-           : mode == TB_STORE ? tb_pass<FDO, P2, TB_STORE, MAXT>
-                              : tb_pass<FDO, P2, TB_FWD, MAXT>;
-}
-template <bool P2, int MAXT>
-static TbFn tb_pick(int fdo, int mode)
-{
-    switch (fdo) {
-    case 2: return tb_mode<2, P2, MAXT>(mode);
-    case 4: return tb_mode<4, P2, MAXT>(mode);
-    case 6: return tb_mode<6, P2, MAXT>(mode);
-    case 8: return tb_mode<8, P2, MAXT>(mode);
-    default: return nullptr;
-    }
-}
-
-template <int MAXT>
-static TbFn tb_p2(const TbProblem &pb)
-{
-    return pb.p2 ? tb_pick<true, MAXT>(pb.fdorder, pb.mode) : tb_pick<false, MAXT>(pb.fdorder, pb.mode);
-}
 static TbFn tb_fn(const TbProblem &pb, int nthr)
 {
-    return nthr <= TB_FEW_THREADS   ? tb_p2<TB_FEW_THREADS>(pb)
-           : nthr <= TB_MID_THREADS ? tb_p2<TB_MID_THREADS>(pb)
-                                    : tb_p2<TB_MAX_THREADS>(pb);
+    switch (pb.fdorder) {
+    case 2: return tb_kernel_fd2(pb.mode, pb.p2, nthr);
+    case 4: return tb_kernel_fd4(pb.mode, pb.p2, nthr);
+    case 6: return tb_kernel_fd6(pb.mode, pb.p2, nthr);
+    case 8: return tb_kernel_fd8(pb.mode, pb.p2, nthr);
+    default: return nullptr;
+    }
 }
 
 static int env_int(const char *name, int lo, int hi)

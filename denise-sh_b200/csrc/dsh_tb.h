@@ -7,6 +7,14 @@
 #include "dsh_tblock.cuh"
 
 namespace dsh {
+/* the kernel of one build: each order is a module of its own, loaded when it is
+ * first needed */
+using TbFn = void (*)(StepArgs, TbGeom, TbExchange, int, int);
+TbFn tb_kernel_fd2(int mode, bool p2, int nthr);
+TbFn tb_kernel_fd4(int mode, bool p2, int nthr);
+TbFn tb_kernel_fd6(int mode, bool p2, int nthr);
+TbFn tb_kernel_fd8(int mode, bool p2, int nthr);
+
 /* what decides whether and how the kernel serves a pass of an elastic context */
 struct TbProblem {
     int fdorder, p2, mode, nx, ny, fw;
