@@ -146,8 +146,9 @@ __global__ void __launch_bounds__(BX *BY, 2) s_multi_p(const __grid_constant__ M
 /* Register classes.  A kernel that holds every body needs the registers of
  * the largest one (FDORDER 8, L 2: 128 per thread, 16 warps per SM) for all
  * its blocks, elastic FDORDER-4 tiles included.  A class kernel holds the
- * body of one key alone and a register budget of its own (velocity: that of
- * the single-model kernel, 64 registers, 32 warps per SM; stress: below),
+ * body of one key alone and a register budget of its own (velocity: 80
+ * registers, 24 warps per SM; 64 and 32 run the same time, 43.5 ms for the
+ * eight-model batch and 20.1 for one of grids up to 700 x 250; stress: below),
  * and the batch launches one per key present, back to back: every grid waits
  * for its predecessor (pdl_wait) before it reads stresses or velocities, so
  * the launches of one half-step run in order and the next one may begin its

@@ -4,7 +4,7 @@
  * with overlapped tiles, FDORDER 2-8).
  *
  * On a grid of less than one wave of blocks the kernel pair's two launches
- * per step are all latency (4.0 us per step at 160 x 80, 4.5 at 500 x 200,
+ * per step are all latency (4.0 us per step at 160 x 80, 4.4 at 500 x 200,
  * of which launches and dependent loads from L2 are 3.0).  Here the grid is
  * cut into one tile per SM and a thread block keeps its tile in shared memory
  * and registers for the whole pass.
@@ -26,9 +26,11 @@
  * writes round n+1 has seen round n of its neighbours, who have read round
  * n-1 by then.  All blocks are resident (cooperative launch).
  *
- * What bounds it: per step about 160 instructions per vector of four points
- * (shared taps, independent chains), per round one exchange of ~2 us through
- * L2.  The launch shape (tw, th, k) minimises that cost (tb_config).
+ * What bounds it: the two barriers of a step (217 to 238 instructions per warp
+ * and step; of 15 to 19 cycles between two instructions of a warp 9 to 11 are
+ * spent at a barrier) and per round one exchange of 2.8 us through L2.  The
+ * launch shape (tw, th, k) minimises that cost (tb_config).  us per step,
+ * pair and this pass: 160 x 80, FDORDER 4: 4.0 and 1.9; 500 x 200: 4.4 and 2.5.
  *
  * Modes: plain forward (TB_FWD; with the energy sum where the pass keeps
  * checkpoints), forward with storage of the acceleration and the strain rates

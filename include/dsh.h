@@ -182,12 +182,15 @@ int dsh_profile_step(dsh_ctx *ctx, int pass, int nsteps, float *out_ms3);
  * per pass of plain elastic forward modelling with the wavefield and model
  * held in the shared memory of one 16-CTA (or 8-CTA) thread-block cluster
  * per shot (FDORDER <= 8, grids whose ceil(NY/16)-row strips fit one CTA's
- * shared memory, e.g. 500 x 200), 5 plain elastic forward modelling with k
- * time steps per launch (FDORDER 2/4/6/8: k = 8/4/3/2), each thread block
- * advancing a tile 32 points wide (and 8-64 rows high, so that all tiles run
- * in one wave where they can) and a recomputed halo of k*(FDORDER-1) points
- * in its shared memory (FDORDER <= 8, NX and NY >= 2 FW, at most 32 source
- * points, 4 sources per point and 512 receivers per shot). */
+ * shared memory, e.g. 500 x 200), 5 one launch per elastic pass (forward,
+ * forward with storage, adjoint) of grids whose tiles run at once, one per
+ * SM: each thread block keeps a tile 32 or 64 points wide and a recomputed
+ * halo of k*(FDORDER-1) points in registers and shared memory and exchanges
+ * its halo with the neighbouring tiles every k steps (k up to 8/4/3/2 for
+ * FDORDER 2/4/6/8; NX and NY >= 2 FW, at most 1024 source points, 8 sources
+ * per point and 2048 receivers per shot).  Without a choice, variant 5 serves
+ * the passes it can up to 262144 points over the shots of a launch where k
+ * >= 2, and 0 the others. */
 #define DSH_STEP_VARIANTS 6
 
 /* Step-kernel autotuner: times nsteps plain forward steps of every variant
