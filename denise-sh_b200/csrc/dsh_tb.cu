@@ -54,12 +54,16 @@ bool tb_config(const TbProblem &pb, TbCfg *cfg)
         const long long tiles = (long long)g.ntx * g.nty * pb.nb;
         const long long bytes = 4LL * tb_smem(g, H, pb.mode).total;
         if (g.nthr > TB_MAX_THREADS || tiles > nsm || bytes > maxsm) return false;
-        /* per step one vector of a thread, slower with the fewer registers of
-           larger blocks, per round the exchange (us; 160 x 80, 448 threads: 1.2 +
-           2.8 / k, 500 x 200, 672 threads: 1.9 + 2.8 / k; one build with 64
-           registers: 1.5 and 2.1) */
-        const double few = g.nthr <= TB_FEW_THREADS ? 1.0 : g.nthr <= TB_MID_THREADS ? 1.05 : 1.2;
-        const double step = 0.5 + 0.0018 * g.nthr * few, t = step + 2.8 / k;
+        /* us: per step one vector of a thread, slower with the fewer registers of
+           larger blocks (the storing and adjoint modes spill more there), per
+           round the exchange, longer among more tiles; fitted to 60 shapes of
+           FDORDER 4, 6 and 8, 50 to 144 tiles, 384 to 1024 threads, 0.13 rms.
+           Against one rate per thread and 2.8 per round: 600 x 250, FDORDER 4: 3.46 ->
+           3.21; 14 shots of 160 x 80: 3.65 -> 3.32; FDORDER 6, 8 shots: 4.22 -> 3.93, 500
+           x 200: 3.80 -> 3.39 */
+        const double large = pb.mode == TB_FWD ? 0.0023 : 0.0028;
+        const double per = g.nthr <= TB_FEW_THREADS ? 0.0012 : g.nthr <= TB_MID_THREADS ? 0.0019 : large;
+        const double t = 0.1 + per * g.nthr + (3.85 + 0.0069 * (double)tiles) / k;
         if (best == 0.0 || t < best) {
             best = t;
             c.geo = g;
