@@ -28,7 +28,7 @@
  *
  * What bounds it: the two barriers of a step (217 to 238 instructions per warp
  * and step; of 15 to 19 cycles between two instructions of a warp 9 to 11 are
- * spent at a barrier) and per round one exchange of 2.8 us through L2.  The
+ * spent at a barrier) and per round one exchange of 4 to 5 us through L2.  The
  * launch shape (tw, th, k) minimises that cost (tb_config).  us per step,
  * pair and this pass: 160 x 80, FDORDER 4: 4.0 and 1.9; 500 x 200: 4.4 and 2.5.
  *

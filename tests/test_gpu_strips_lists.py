@@ -90,6 +90,29 @@ def test_variants_agree_with_the_pair(variant):
         assert all(np.array_equal(a, b) for a, b in zip(got, ref))
 
 
+@pytest.mark.parametrize("fdo,k,rows", [(4, 4, 8), (4, 4, 16), (4, 4, 40), (4, 4, 48), (8, 2, 8), (8, 2, 32), (2, 8, 8),
+                                        (6, 3, 8), (6, 2, 48)])
+def test_blocked_pass_of_each_block_size(fdo, k, rows, monkeypatch):
+    """Blocks of 448, 576, 896, 1024 (FDORDER 4), 576, 960 (8), 288 (2), 608 and 960 (6) threads: the three builds in the
+    forward, storing and adjoint modes against the kernel pair."""
+    monkeypatch.setenv("DSH_TB_STEPS", str(k))
+    monkeypatch.setenv("DSH_TB_ROWS", str(rows))
+    kw, vs, rho, _, shots = _case(203, 97, 10, fdo, 0, 1, 0.6, 1.0, 40, seed=fdo)
+    res = []
+    with dsh.Engine(dsh.make_params(max_shots=1, **kw)) as e:
+        e.set_model(vs, rho)
+        for variant in (0, 5):
+            e.set_step_variant(variant)
+            seis = e.forward(shots)
+            launches = e.stats()["kernel_launches"]
+            g = e.gradient(shots, [x * np.float32(0.6) for x in seis])
+            res.append((seis, g["g_vs"], g["g_rho"], g["l2"], launches))
+    (s0, *g0, n0), (s5, *g5, n5) = res
+    assert all(np.array_equal(a, b) for a, b in zip(s0, s5))
+    assert all(np.array_equal(a, b) for a, b in zip(g0, g5))
+    assert n5 < kw["nt"] < n0               # one launch per pass: the blocked pass ran
+
+
 def test_uneven_batch():
     members = [_case(*c, seed=7) for c in (CASES[0], (45, 37, 18, 8, 2, 0, 0.6, 1.5, 20), (262, 19, 5, 8, 0, 1, 0.5, 3.0, 131))]
     with dsh.Batch([dsh.make_params(max_shots=3, **m[0]) for m in members]) as b:
