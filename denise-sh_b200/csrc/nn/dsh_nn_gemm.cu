@@ -246,18 +246,20 @@ __global__ void __launch_bounds__(THREADS, 1)
             for (int c = 0; c < BN; c += 16) {
                 float v[16];
                 tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-                if (row >= g.M) continue;
-                const int nb = n0 + c;
+                if (row < g.M) {
+                    const int nb = n0 + c;
 #pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const int n = nb + k;
-                    if (n >= g.N) break;
-                    float x = v[k];
-                    if (g.bias) x += g.bias[n];
-                    if (g.relu) x = fmaxf(x, 0.0f);
-                    if (c32) c32[(long long)row * g.ldc + n] = x;
-                    if (g.c16) g.c16[(long long)row * g.ldc + n] = __float2bfloat16_rn(x);
+                    for (int k = 0; k < 16; k++) {
+                        const int n = nb + k;
+                        if (n >= g.N) break;
+                        float x = v[k];
+                        if (g.bias) x += g.bias[n];
+                        if (g.relu) x = fmaxf(x, 0.0f);
+                        if (c32) c32[(long long)row * g.ldc + n] = x;
+                        if (g.c16) g.c16[(long long)row * g.ldc + n] = __float2bfloat16_rn(x);
+                    }
                 }
+                __syncwarp();                         /* rows past M stored nothing: together again for the next load */
             }
         } else if (lane == 0) {                      /* any warp whose wait expired reports it */
             atomicExch(g.err, DSH_NN_ERR_TIMEOUT);
@@ -393,28 +395,30 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int c = 0; c < BN && n0 + c < g.N; c += 16) {
             float v[16];
             tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-            if (!in) continue;
             const int nb = n0 + c;
+            if (in) {
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                if (g.bias && nb + k < g.N) v[k] += g.bias[nb + k];
-                if (g.relu) v[k] = fmaxf(v[k], 0.0f);
-            }
-#pragma unroll
-            for (int h = 0; h < 16; h += 8) {         /* N is a multiple of 8 */
-                if (nb + h >= g.N) break;
-                if (g.c32) {
-                    float4 *o = reinterpret_cast<float4 *>(g.c32 + row + nb + h);
-                    o[0] = make_float4(v[h], v[h + 1], v[h + 2], v[h + 3]);
-                    o[1] = make_float4(v[h + 4], v[h + 5], v[h + 6], v[h + 7]);
+                for (int k = 0; k < 16; k++) {
+                    if (g.bias && nb + k < g.N) v[k] += g.bias[nb + k];
+                    if (g.relu) v[k] = fmaxf(v[k], 0.0f);
                 }
-                if (g.c16) {
-                    __nv_bfloat162 q[4];
 #pragma unroll
-                    for (int e = 0; e < 4; e++) q[e] = __floats2bfloat162_rn(v[h + 2 * e], v[h + 2 * e + 1]);
-                    *reinterpret_cast<uint4 *>(g.c16 + row + nb + h) = *reinterpret_cast<const uint4 *>(q);
+                for (int h = 0; h < 16; h += 8) {     /* N is a multiple of 8 */
+                    if (nb + h >= g.N) break;
+                    if (g.c32) {
+                        float4 *o = reinterpret_cast<float4 *>(g.c32 + row + nb + h);
+                        o[0] = make_float4(v[h], v[h + 1], v[h + 2], v[h + 3]);
+                        o[1] = make_float4(v[h + 4], v[h + 5], v[h + 6], v[h + 7]);
+                    }
+                    if (g.c16) {
+                        __nv_bfloat162 q[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) q[e] = __floats2bfloat162_rn(v[h + 2 * e], v[h + 2 * e + 1]);
+                        *reinterpret_cast<uint4 *>(g.c16 + row + nb + h) = *reinterpret_cast<const uint4 *>(q);
+                    }
                 }
             }
+            __syncwarp();                             /* pixels outside the map stored nothing: together for the next load */
         }
     } else if (lane == 0) {
         atomicExch(g.err, DSH_NN_ERR_TIMEOUT);

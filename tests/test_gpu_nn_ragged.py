@@ -1,0 +1,58 @@
+"""Epilogues of the tensor-core GEMM and of the implicit convolution where some lanes of a warp have nothing to store: rows
+past M, pixels outside the map (a warp holds 2 rows x 16 columns), with several 16-column tensor-memory loads per warp,
+against 64-bit products of the same bf16 operands.  Tolerance: K products added in float, each addition off by at most
+2^-23 of the running sum, which never exceeds the sum of the magnitudes; as much again for the bias and the output."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(got, ref, mag, K):
+    assert bool(((got.double() - ref).abs() <= (K + 2) * 2.0 ** -23 * mag).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 48, 64), (33, 96, 72), (77, 288, 128), (129, 64, 64), (255, 256, 136)])
+def test_gemm_rows_past_the_last(M, N, K):
+    import torch
+
+    from dsh import nn as dnn
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    A, B = (torch.randn(n, K, device="cuda", generator=g).bfloat16() for n in (M, N))
+    bias = torch.randn(N, device="cuda", generator=g)
+    c32 = torch.full((M + 3, N), 7.0, device="cuda")
+    ctx = dnn.Ctx(torch)
+    ctx.gemm(M, N, K, A, K, B, K, c32=c32, bias=bias)
+    ctx.check()
+    _check(c32[:M], A.double() @ B.double().t() + bias.double(),
+           A.double().abs() @ B.double().abs().t() + bias.double().abs(), K)
+    assert bool((c32[M:] == 7).all())
+
+
+@pytest.mark.parametrize("B,H,W,C,N", [(1, 1, 1, 32, 48), (1, 3, 5, 64, 96), (2, 9, 15, 32, 256), (1, 7, 17, 128, 64),
+                                       (1, 25, 31, 96, 288)])
+def test_convolution_pixels_outside_the_map(B, H, W, C, N):
+    import torch
+
+    from dsh import nn as dnn
+
+    g = torch.Generator(device="cuda").manual_seed(H * W)
+    P, K = B * H * W, 9 * C
+    x = torch.randn(P, C, device="cuda", generator=g).bfloat16()
+    w = torch.randn(N, 9, C, device="cuda", generator=g).bfloat16()
+    bias = torch.randn(N, device="cuda", generator=g)
+    c32 = torch.full((P + 3, N), 7.0, device="cuda")
+    ctx = dnn.Ctx(torch)
+    ctx.conv3x3(x, B, H, W, C, w, K, N, c32=c32, bias=bias)
+    ctx.check()
+
+    def conv(xd, wd, bd):
+        pad = torch.nn.functional.pad(xd.view(B, H, W, C), (0, 0, 1, 1, 1, 1))
+        out = bd.expand(P, N).clone()
+        for t in range(9):
+            out += pad[:, t // 3:t // 3 + H, t % 3:t % 3 + W].reshape(P, C) @ wd[:, t].t()
+        return out
+
+    xd, wd, bd = x.double(), w.double(), bias.double()
+    _check(c32[:P], conv(xd, wd, bd), conv(xd.abs(), wd.abs(), bd.abs()), K)
+    assert bool((c32[P:] == 7).all())
