@@ -117,6 +117,12 @@ class Ctx:
         _ck(nnlib().dsh_nn_gemm(M, N, K, _p(A), lda, _p(B), ldb, _p(c32), _p(c16), ldc, _p(bias), int(relu),
                                 splits, _p(part), int(accumulate), _p(self.err), self.st), "dsh_nn_gemm")
 
+    @staticmethod
+    def conv3x3_ok(x, C, N, out):
+        """Whether dsh_nn_conv3x3 takes the call: whole K blocks of 32 channels, 16-byte rows of the output, aligned
+        bases.  Other channel counts and offset tensors go through columns and the GEMM."""
+        return C % 32 == 0 and N % 8 == 0 and x.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
+
     def conv3x3(self, x, B, H, W, C, w, ldw, N, c32=None, c16=None, bias=None, relu=False):
         _ck(nnlib().dsh_nn_conv3x3(_p(x), B, H, W, C, _p(w), ldw, N, _p(c32), _p(c16), _p(bias), int(relu), _p(self.err),
                                    self.st), "dsh_nn_conv3x3")
@@ -157,7 +163,7 @@ class Conv3x3:
         """x bf16 [P][cin] -> y bf16 [P][cout] (ReLU applied)."""
         ctx = self.ctx
         P = B * H * W
-        if self.cin % 32 == 0:
+        if ctx.conv3x3_ok(x, self.cin, self.cout, y):
             ctx.conv3x3(x, B, H, W, self.cin, self.wb, self.ldk, self.cout, c16=y, bias=self.b, relu=True)
             return
         col = ctx.scratch("col", P * self.ldk, ctx.torch.bfloat16)
@@ -181,7 +187,7 @@ class Conv3x3:
         _ck(nnlib().dsh_nn_transpose(_p(dz), P, self.cout, _p(dzT), ldp, ctx.st), "transpose")
         splits = max(1, min(64, P // 8192))
         ctx.gemm(self.K, self.cout, P, colT, ldp, dzT, ldp, c32=self.gwt, splits=splits, accumulate=True)
-        if dx is not None and self.cout % 32 == 0:
+        if dx is not None and ctx.conv3x3_ok(dz, self.cout, self.cin, dx):
             ctx.conv3x3(dz, B, H, W, self.cout, self.wf, self.ldf, self.cin, c32=dx)
         elif dx is not None:
             col = ctx.scratch("col", P * self.ldf, torch.bfloat16)

@@ -56,3 +56,47 @@ def test_convolution_pixels_outside_the_map(B, H, W, C, N):
     xd, wd, bd = x.double(), w.double(), bias.double()
     _check(c32[:P], conv(xd, wd, bd), conv(xd.abs(), wd.abs(), bd.abs()), K)
     assert bool((c32[P:] == 7).all())
+
+
+@pytest.mark.parametrize("cin,cout,off", [(32, 12, 0), (12, 32, 0), (32, 5, 0), (64, 32, 0), (32, 32, 1), (40, 64, 1)])
+def test_conv_layer_of_any_channel_counts(cin, cout, off):
+    """A layer's forward and backward pass where the implicit convolution does not apply (output channels no multiple of 8,
+    tensors off a 16-byte boundary) and where it does."""
+    import numpy as np
+    import torch
+
+    from dsh import nn as dnn
+
+    B, H, W = 2, 5, 9
+    P, K = B * H * W, 9 * cin
+    g = torch.Generator(device="cuda").manual_seed(cin + cout)
+    ctx = dnn.Ctx(torch)
+    layer = dnn.Conv3x3(ctx, cin, cout, np.random.default_rng(cout))
+    layer.b.copy_(torch.randn(cout, device="cuda", generator=g))
+    x = torch.empty(P * cin + off, dtype=torch.bfloat16, device="cuda")[off:]
+    y = torch.empty(P * cout + off, dtype=torch.bfloat16, device="cuda")[off:]
+    dy, dx = (torch.empty(P * c + off, device="cuda")[off:] for c in (cout, cin))
+    x.copy_(torch.randn(P * cin, device="cuda", generator=g))
+    dy.copy_(torch.randn(P * cout, device="cuda", generator=g))
+    dy0 = dy.double()
+    layer.zero_grad()
+    layer.forward(x, B, H, W, y)
+    layer.backward(x, y, dy, B, H, W, dx=dx)
+    ctx.check()
+    w = layer.w.bfloat16().double().view(cout, 3, 3, cin).permute(0, 3, 1, 2)
+    conv = torch.nn.functional.conv2d
+    maps = lambda t, c: t.view(B, H, W, c).permute(0, 3, 1, 2)
+    flat = lambda t, c: t.permute(0, 2, 3, 1).reshape(P, c)
+    xd = maps(x.double(), cin)
+    z, mag = flat(conv(xd, w, layer.b.double(), padding=1), cout), flat(conv(xd.abs(), w.abs(), layer.b.double().abs(), padding=1), cout)
+    got = y.view(P, cout).double()
+    assert bool(((got - z.clamp(min=0)).abs() <= 2.0 ** -8 * z.abs() + 2 * (K + 2) * 2.0 ** -23 * mag).all())
+    dz32 = torch.where(y.double() > 0, dy0, torch.zeros_like(dy0))
+    dz = maps(dz32.bfloat16().double(), cout)
+    wt = w.flip(2, 3).transpose(0, 1)
+    _check(dx.view(P, cin), flat(conv(dz, wt, padding=1), cin), flat(conv(dz.abs(), wt.abs(), padding=1), cin), 9 * cout)
+    xp = torch.nn.functional.pad(x.double().view(B, H, W, cin), (0, 0, 1, 1, 1, 1))
+    col = torch.cat([xp[:, t // 3:t // 3 + H, t % 3:t % 3 + W].reshape(P, cin) for t in range(9)], 1)
+    dzf = flat(dz, cout)
+    _check(layer.gwt.view(K, cout), col.t() @ dzf, col.abs().t() @ dzf.abs(), P)
+    _check(layer.gb, dz32.view(P, cout).sum(0), dz32.view(P, cout).abs().sum(0), P)
