@@ -622,7 +622,7 @@ extern "C" dsh_ctx *dsh_create(const dsh_params *p, int device, int *status)
 namespace dsh::eng {
 void drop_graphs(dsh_ctx *ctx)
 {
-    for (auto &kv : ctx->graphs) cudaGraphExecDestroy(kv.second);
+    for (auto &kv : ctx->graphs) cudaGraphExecDestroy(kv.second.exec);
     ctx->graphs.clear();
 }
 }  // namespace dsh::eng
@@ -1523,7 +1523,7 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
     return DSH_OK;
 }
 
-static int get_graph(dsh_ctx *ctx, Pass pass, int nb, int K, cudaGraphExec_t *out)
+static int get_graph(dsh_ctx *ctx, Pass pass, int nb, int K, StepGraph *out)
 {
     const long long vcode = v_code(ctx);
     const long long key = ((long long)pass << 52) | ((long long)ctx->fused_inject << 51) |
@@ -1532,17 +1532,16 @@ static int get_graph(dsh_ctx *ctx, Pass pass, int nb, int K, cudaGraphExec_t *ou
     auto it = ctx->graphs.find(key);
     if (it != ctx->graphs.end()) { *out = it->second; return DSH_OK; }
     cudaGraph_t g;
-    long long nl = 0;
+    StepGraph sg;
     CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
-    int rc = launch_step_chunk(ctx, pass, nb, K, &nl);
+    int rc = launch_step_chunk(ctx, pass, nb, K, &sg.launches);
     cudaError_t e = cudaStreamEndCapture(ctx->st, &g);
     if (rc != DSH_OK) return rc;
     CK(e);
-    cudaGraphExec_t exec;
-    CK(cudaGraphInstantiate(&exec, g, 0));
+    CK(cudaGraphInstantiate(&sg.exec, g, 0));
     cudaGraphDestroy(g);
-    ctx->graphs[key] = exec;
-    *out = exec;
+    ctx->graphs[key] = sg;
+    *out = sg;
     return DSH_OK;
 }
 
@@ -1762,7 +1761,6 @@ static int run_steps(dsh_ctx *ctx, Pass pass, int nb, int n0, int count)
     const int K = std::min(ctx->chunk, count);
     const int nfull = count / K, rem = count % K;
     const bool fused = use_fused(ctx, pass);
-    const long long per_step = fused ? 1 : ctx->fused_inject ? 2 : 3;
     /* the fused step leaves the state of step n in buffer n & 1 */
     if (pass != P_RECOMP) ctx->state_b = fused ? ((n0 + count - 1) & 1) : 0;
     set_int_kernel<<<1, 1, 0, ctx->st>>>(ctx->d_nt, n0);
@@ -1777,13 +1775,13 @@ static int run_steps(dsh_ctx *ctx, Pass pass, int nb, int n0, int count)
         }
         return DSH_OK;
     }
-    cudaGraphExec_t full, tail = nullptr;
+    StepGraph full, tail;
     int rc = get_graph(ctx, pass, nb, K, &full);
     if (rc != DSH_OK) return rc;
     if (rem && (rc = get_graph(ctx, pass, nb, rem, &tail)) != DSH_OK) return rc;
-    for (int c = 0; c < nfull; c++) CK(cudaGraphLaunch(full, ctx->st));
-    if (rem) CK(cudaGraphLaunch(tail, ctx->st));
-    ctx->launches += (per_step * K + 1) * nfull + (rem ? per_step * rem + 1 : 0);
+    for (int c = 0; c < nfull; c++) CK(cudaGraphLaunch(full.exec, ctx->st));
+    if (rem) CK(cudaGraphLaunch(tail.exec, ctx->st));
+    ctx->launches += full.launches * nfull + tail.launches;
     return DSH_OK;
 }
 

@@ -18,6 +18,12 @@ namespace dsh {
 enum Pass { P_FWD_PLAIN = 0, P_FWD_STORE = 1, P_FWD_HESS = 2, P_ADJ = 3, P_FWD_CKPT = 4, P_RECOMP = 5 };
 }  // namespace dsh
 
+/* a captured chunk of steps and the kernels it launches */
+struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    long long launches = 0;
+};
+
 struct dsh_ctx {
     dsh_params p;
     int dev = 0;
@@ -102,7 +108,7 @@ struct dsh_ctx {
     float *d_taper_box = nullptr;
     void *d_taper_shot = nullptr;         /* S x TaperShot */
     std::vector<double> shot_l2;          /* per-shot L2 misfits of the last gradient */
-    std::map<long long, cudaGraphExec_t> graphs;
+    std::map<long long, StepGraph> graphs;
     cudaEvent_t ev[4];
     cudaEvent_t ev_wait = nullptr;        /* recorded by the bounded host waits (timing disabled) */
     double host_timeout_s = 1800.0;       /* wall-clock limit of every host wait (dsh_set_wait_limits) */
