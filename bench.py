@@ -495,7 +495,9 @@ def c3_sub(a, local):
         "gpu_launches": launches,
         "l2": f"inputs larger than L2 (state of {nsh} shots {(3 + 2 * 2) * n * 4 * nsh / 1e6:.0f} MB)",
         "roofline": {"bound": "hbm", "achieved": s_gbs, "peak": hbm, "unit": "GB/s", "frac": s_gbs / hbm,
-                     "kernel": "s_step<8,2> (forward pass with storage, 64 slots)", "bytes_per_point": ks,
+                     "kernel": "s_step<8,2> (forward pass with storage: a half-step of all 64 slots, in the launches "
+                               "of a pass; counted bytes, those of a group's wavefield mostly from L2)",
+                     "bytes_per_point": ks,
                      "ms_per_launch": prof["s_step"], "peak_source": peak_kind},
         "kernels_ms": prof, "v_step_gbs": v_gbs,
         "clocks": clk,

@@ -1439,9 +1439,17 @@ static int side_stream(cudaStream_t *st, cudaEvent_t *e0, cudaEvent_t *e1, dsh_c
     return DSH_OK;
 }
 
-static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chunk, long long *nlaunch, int slot0 = 0)
+/* the kernel pair of a pass for nb slots: kernels, arguments and launch shapes */
+struct PairLaunch {
+    KFn vk, sk;
+    VPick vp;
+    StepArgs sa;
+    dim3 vgrid, vblock, sgrid, sblock;       /* z: slots of a launch (v_step_tp: slots in y) */
+    int half;                                /* slot_split */
+};
+
+static int pair_launch(dsh_ctx *ctx, Pass pass, int nb, PairLaunch *l)
 {
-    if (use_fused(ctx, pass)) return launch_fused_chunk(ctx, pass, nb, nsteps_in_chunk, nlaunch);
     const dsh_params &p = ctx->p;
     int vflags = 0, sflags = 0;
     switch (pass) {
@@ -1454,23 +1462,34 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
     }
     if (p.grad_q && (sflags == SF_STRAIN_OUT || sflags == SF_CORR))   /* the Qs gradient's two halves */
         sflags |= sflags == SF_CORR ? SF_CORRQ : SF_QSENS;
-    const VPick vp = pick_v(ctx, p.fdorder, vflags, dh_pow2(p.dh));
-    KFn vk = vp.k, sk = s_kernel(p.fdorder, p.l, sflags);
-    if (!vk || !sk) return DSH_ERR_PARAM;
-    StepArgs sa = step_args(ctx, pass);
-    InjectArgs ia = inject_args(ctx, pass);
+    l->vp = pick_v(ctx, p.fdorder, vflags, dh_pow2(p.dh));
+    l->vk = l->vp.k;
+    l->sk = s_kernel(p.fdorder, p.l, sflags);
+    if (!l->vk || !l->sk) return DSH_ERR_PARAM;
+    l->sa = step_args(ctx, pass);
     const int sr = s_rows();
-    dim3 block(BX, sr, 1);
-    dim3 grid((unsigned)((p.nx + 4 * BX - 1) / (4 * BX)), (unsigned)((p.ny + sr - 1) / sr), (unsigned)nb);
-    if (sa.tl.on && sa.tl.sample) {          /* the stress launch samples the receivers (sample_block) */
-        sa.tl.samp_by = (int)grid.y;
-        sa.tl.sample = 0;
-        sa.tl.row0 = ctx->rows_f[0];
-        sa.tl.row1 = ctx->rows_f[1];
-        grid.y += 1;
+    l->sblock = dim3(BX, sr, 1);
+    l->sgrid = dim3((unsigned)((p.nx + 4 * BX - 1) / (4 * BX)), (unsigned)((p.ny + sr - 1) / sr), (unsigned)nb);
+    TileLists &tl = l->sa.tl;
+    if (tl.on && tl.sample) {                /* the stress launch samples the receivers (sample_block) */
+        tl.samp_by = (int)l->sgrid.y;
+        tl.sample = 0;
+        tl.row0 = ctx->rows_f[0];
+        tl.row1 = ctx->rows_f[1];
+        l->sgrid.y += 1;
     }
-    dim3 vgrid, vblock;
-    v_shape(ctx, vp, nb, &vgrid, &vblock);
+    v_shape(ctx, l->vp, nb, &l->vgrid, &l->vblock);
+    l->half = slot_split(ctx, l->vp, nb);
+    return DSH_OK;
+}
+
+static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chunk, long long *nlaunch, int slot0 = 0)
+{
+    if (use_fused(ctx, pass)) return launch_fused_chunk(ctx, pass, nb, nsteps_in_chunk, nlaunch);
+    PairLaunch l;
+    const int rc = pair_launch(ctx, pass, nb, &l);
+    if (rc != DSH_OK) return rc;
+    InjectArgs ia = inject_args(ctx, pass);
     /* velocity and stress kernels overlap their prologues with the
      * predecessor through programmatic dependent launch; the first velocity
      * kernel of a chunk follows the step-counter update and is launched plainly */
@@ -1478,12 +1497,10 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
     cfg.dynamicSmemBytes = 0;
     cfg.stream = ctx->st;
     static const bool use_pdl = getenv("DSH_NO_PDL") == nullptr;
-    const int half = slot_split(ctx, vp, nb);
+    const int half = l.half;
     if (half) {
         CK(cudaEventRecord(ctx->ev_fork, ctx->st));
         CK(cudaStreamWaitEvent(ctx->st2, ctx->ev_fork, 0));
@@ -1493,23 +1510,23 @@ static int launch_step_chunk(dsh_ctx *ctx, Pass pass, int nb, int nsteps_in_chun
         cfg.stream = part ? ctx->st2 : ctx->st;
         for (int k = 0; k < nsteps_in_chunk; k++) {
             int off = launch_word(k, s0);
-            void *args[2] = {&sa, &off};
+            void *args[2] = {&l.sa, &off};
             cfg.attrs = (use_pdl && k > 0) ? &attr : nullptr;
             cfg.numAttrs = (use_pdl && k > 0) ? 1 : 0;
-            cfg.gridDim = vgrid;
+            cfg.gridDim = l.vgrid;
             if (half || slot0) cfg.gridDim.z = (unsigned)ns;
-            cfg.blockDim = vblock;
-            CK(cudaLaunchKernelExC(&cfg, (const void *)vk, args));
-            cfg.gridDim = dim3(grid.x, grid.y, (unsigned)ns);
-            cfg.blockDim = block;
-            if (!sa.tl.on) {
+            cfg.blockDim = l.vblock;
+            CK(cudaLaunchKernelExC(&cfg, (const void *)l.vk, args));
+            cfg.gridDim = dim3(l.sgrid.x, l.sgrid.y, (unsigned)ns);
+            cfg.blockDim = l.sblock;
+            if (!l.sa.tl.on) {
                 void *iargs[2] = {&ia, &off};
                 CK(cudaLaunchKernel((const void *)inject_sample, dim3(nb), dim3(128), iargs, 0, ctx->st));
                 *nlaunch += 1;
             }
             cfg.attrs = use_pdl ? &attr : nullptr;
             cfg.numAttrs = use_pdl ? 1 : 0;
-            CK(cudaLaunchKernelExC(&cfg, (const void *)sk, args));
+            CK(cudaLaunchKernelExC(&cfg, (const void *)l.sk, args));
             *nlaunch += 2;
         }
     }
@@ -1734,9 +1751,9 @@ static int run_groups(dsh_ctx *ctx, Pass pass, int nb, int n0, int count, int gr
     for (int s0 = 0; s0 < nb; s0 += group) {
         set_int_kernel<<<1, 1, 0, ctx->st>>>(ctx->d_nt, n0);
         ctx->launches += 1;
-        for (int done = 0; done < count; done += 0x7000) {
+        for (int done = 0; done < count; done += WORD_STEPS) {
             long long nl = 0;
-            const int rc = launch_step_chunk(ctx, pass, std::min(group, nb - s0), std::min(0x7000, count - done), &nl, s0);
+            const int rc = launch_step_chunk(ctx, pass, std::min(group, nb - s0), std::min(WORD_STEPS, count - done), &nl, s0);
             if (rc != DSH_OK) return rc;
             ctx->launches += nl;
         }
@@ -2503,54 +2520,60 @@ extern "C" int dsh_profile_step(dsh_ctx *ctx, int pass, int nsteps, float *out_m
     if (ctx->ckpt_c && (pass == P_FWD_STORE || pass == P_ADJ) && nsteps > ctx->ckpt_c) nsteps = ctx->ckpt_c;
     if (!ctx->model_set || ctx->ntr_b.empty() || ((pass == P_FWD_STORE || pass == P_ADJ) && !ctx->fwd)) return DSH_ERR_STATE;
     CK(cudaSetDevice(ctx->dev));
-    const dsh_params &p = ctx->p;
+    nsteps = std::min(nsteps, WORD_STEPS);
     const int nb = (int)ctx->ntr_b.size();
-    int vflags = 0, sflags = 0;
-    if (pass == P_FWD_STORE) sflags = SF_STRAIN_OUT;
-    if (pass == P_FWD_HESS) { vflags = VF_HESS; sflags = SF_HESS; }
-    if (pass == P_ADJ) { vflags = VF_ADJOINT | VF_CORR; sflags = SF_CORR; }
-    const VPick vp = pick_v(ctx, p.fdorder, vflags, dh_pow2(p.dh));
-    KFn vk = vp.k, sk = s_kernel(p.fdorder, p.l, sflags);
-    if (!vk || !sk) return DSH_ERR_PARAM;
-    StepArgs sa = step_args(ctx, (Pass)pass);
+    int rc = nb > 1 ? side_stream(&ctx->st2, &ctx->ev_fork, &ctx->ev_join, ctx) : DSH_OK;
+    if (rc != DSH_OK) return rc;
+    int group = slot_group(ctx, (Pass)pass, nb);
+    if (!group) group = nb;
     InjectArgs ia = inject_args(ctx, (Pass)pass);
-    const int sr = s_rows();
-    dim3 block(BX, sr, 1);
-    dim3 grid((unsigned)((p.nx + 4 * BX - 1) / (4 * BX)), (unsigned)((p.ny + sr - 1) / sr), (unsigned)nb);
-    dim3 vgrid, vblock;
-    v_shape(ctx, vp, nb, &vgrid, &vblock);
-    /* each kernel launched nsteps times back to back between one event pair */
-    cudaEvent_t ev[6];
+    cudaEvent_t ev[2];
     for (auto &e : ev) CK(cudaEventCreate(&e));
     set_int_kernel<<<1, 1, 0, ctx->st>>>(ctx->d_nt, 1);
-    {   /* one untimed launch of each kernel first (lazy module loading) */
-        int off = 0;
-        void *args[2] = {&sa, &off};
-        void *iargs[2] = {&ia, &off};
-        CK(cudaLaunchKernel((const void *)vk, vgrid, vblock, args, 0, ctx->st));
-        if (!sa.tl.on) CK(cudaLaunchKernel((const void *)inject_sample, dim3(nb), dim3(128), iargs, 0, ctx->st));
-        CK(cudaLaunchKernel((const void *)sk, grid, block, args, 0, ctx->st));
-    }
-    for (int q = 0; q < 3; q++) {
-        CK(cudaEventRecord(ev[2 * q], ctx->st));
-        for (int k = 0; k < nsteps; k++) {
-            int off = k;
-            void *args[2] = {&sa, &off};
-            void *iargs[2] = {&ia, &off};
-            if (q == 0) CK(cudaLaunchKernel((const void *)vk, vgrid, vblock, args, 0, ctx->st));
-            if (q == 1 && !sa.tl.on) CK(cudaLaunchKernel((const void *)inject_sample, dim3(nb), dim3(128), iargs, 0, ctx->st));
-            if (q == 2) CK(cudaLaunchKernel((const void *)sk, grid, block, args, 0, ctx->st));
-        }
-        CK(cudaEventRecord(ev[2 * q + 1], ctx->st));
-    }
-    WAIT(ctx);
     double acc[3] = {0, 0, 0};
-    for (int q = 0; q < 3; q++) {
-        float ms = 0;
-        cudaEventElapsedTime(&ms, ev[2 * q], ev[2 * q + 1]);
-        acc[q] = ms;
+    /* kernel q of the pair for a group of slots, nsteps times back to back, its halves on their two streams */
+    auto repeat = [&](const PairLaunch &l, int q, int g0, int gn, int count) -> int {
+        if (l.half) {
+            CK(cudaEventRecord(ctx->ev_fork, ctx->st));
+            CK(cudaStreamWaitEvent(ctx->st2, ctx->ev_fork, 0));
+        }
+        for (int k = 0; k < count; k++)
+            for (int part = 0; part < (l.half ? 2 : 1); part++) {
+                const int s0 = g0 + (part ? l.half : 0), ns = l.half ? (part ? gn - l.half : l.half) : gn;
+                const cudaStream_t st = part ? ctx->st2 : ctx->st;
+                dim3 vgrid = l.vgrid, sgrid = l.sgrid;
+                if (l.half || g0) vgrid.z = (unsigned)ns;
+                sgrid.z = (unsigned)ns;
+                int off = launch_word(k, s0);
+                void *args[2] = {const_cast<StepArgs *>(&l.sa), &off}, *iargs[2] = {&ia, &off};
+                if (q == 0) CK(cudaLaunchKernel((const void *)l.vk, vgrid, l.vblock, args, 0, st));
+                if (q == 1) CK(cudaLaunchKernel((const void *)inject_sample, dim3(nb), dim3(128), iargs, 0, st));
+                if (q == 2) CK(cudaLaunchKernel((const void *)l.sk, sgrid, l.sblock, args, 0, st));
+            }
+        if (l.half) {
+            CK(cudaEventRecord(ctx->ev_join, ctx->st2));
+            CK(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
+        }
+        return DSH_OK;
+    };
+    for (int g0 = 0; g0 < nb && rc == DSH_OK; g0 += group) {
+        const int gn = std::min(group, nb - g0);
+        PairLaunch l;
+        if ((rc = pair_launch(ctx, (Pass)pass, gn, &l)) != DSH_OK) break;
+        for (int q = 0; q < 3 && rc == DSH_OK; q++) {
+            if (q == 1 && l.sa.tl.on) continue;
+            if ((rc = repeat(l, q, g0, gn, 1)) != DSH_OK) break;       /* untimed (lazy module loading) */
+            cudaEventRecord(ev[0], ctx->st);
+            if ((rc = repeat(l, q, g0, gn, nsteps)) != DSH_OK) break;
+            cudaEventRecord(ev[1], ctx->st);
+            rc = wait_stream(ctx);
+            float ms = 0;
+            cudaEventElapsedTime(&ms, ev[0], ev[1]);
+            acc[q] += ms;
+        }
     }
     for (auto &e : ev) cudaEventDestroy(e);
+    if (rc != DSH_OK) return rc;
     for (int q = 0; q < 3; q++) out_ms3[q] = (float)(acc[q] / nsteps);
     cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->st);   /* repeated steps of one kernel may overflow */
     return check_status(ctx);

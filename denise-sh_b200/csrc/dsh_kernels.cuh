@@ -801,7 +801,8 @@ __device__ __forceinline__ void v_body(const StepArgs &a, int nt_off, int i0, in
 }
 
 /* The launch word of v_step and s_step: the step's offset from the counter in
- * the low 16 bits, the first shot slot of the launch in the high ones. */
+ * the low 16 bits (up to WORD_STEPS), the first shot slot of the launch in the high ones. */
+constexpr int WORD_STEPS = 0x7000;
 __host__ __device__ __forceinline__ int launch_word(int nt_off, int slot0) { return nt_off | (int)((unsigned)slot0 << 16); }
 __device__ __forceinline__ int word_off(int w) { return w & 0xffff; }
 __device__ __forceinline__ int word_slot(int w) { return (int)blockIdx.z + (int)((unsigned)w >> 16); }

@@ -302,7 +302,7 @@ class Engine:
     PASSES = {"forward": 0, "forward_store": 1, "forward_hessian": 2, "adjoint": 3}
 
     def profile_step(self, pass_name: str, nsteps: int) -> dict:
-        """Mean device ms per launch of the velocity, injection and stress kernels."""
+        """Mean device ms per half-step (all launches of it) of the velocity, injection and stress kernels."""
         out = np.zeros(3, np.float32)
         _check(lib().dsh_profile_step(self.h, self.PASSES[pass_name], nsteps, out.ctypes.data), "dsh_profile_step")
         return {"v_step": float(out[0]), "inject_sample": float(out[1]), "s_step": float(out[2])}

@@ -168,9 +168,13 @@ int dsh_set_stream(dsh_ctx *ctx, void *stream);
 
 /* Per-kernel timing: launches each kernel of pass `pass` (0 forward,
  * 1 forward with storage, 2 forward with Hessian sums, 3 adjoint) `nsteps`
- * times back to back on the last batch between one CUDA event pair and
- * returns the mean device time per launch in ms: out[0] velocity step,
- * out[1] separate injection/sampling (0 when fused), out[2] stress step.
+ * times (at most 28672) back to back on the last batch between one CUDA event
+ * pair and returns the mean device time per half-step in ms: out[0] velocity
+ * step, out[1] separate injection/sampling (0 when fused), out[2] stress step.
+ * Where a pass advances its shot slots in groups, each group's launch is
+ * repeated by itself and the means are added; two halves of the slots run on
+ * two streams as in the pass (which also overlaps the velocity launch of one
+ * half with the stress launch of the other).
  * Call it after a dsh_gradient on the same shots; it overwrites the
  * wavefield state, which is rebuilt by the next call. */
 int dsh_profile_step(dsh_ctx *ctx, int pass, int nsteps, float *out_ms3);
