@@ -1652,10 +1652,13 @@ static bool tblock_cfg(dsh_ctx *ctx, Pass pass, int nb, TbProblem *pb, TbCfg *cf
             if (getenv(v)) return true;
         return false;
     }();
-    const bool on = ctx->sel_tblock >= 0 ? ctx->sel_tblock != 0 : env ? atoi(env) != 0 : !other;
+    /* the autotuner chose for plain forward passes: the others keep the rule of an untuned context */
+    const bool tuned = ctx->sel_tuned && pass != P_FWD_PLAIN && (ctx->sel_persist > 0 || ctx->sel_cluster > 0 || ctx->sel_tblock > 0);
+    const int sel = tuned ? -1 : ctx->sel_tblock;
+    const bool on = sel >= 0 ? sel != 0 : env ? atoi(env) != 0 : !other;
     const dsh_params &p = ctx->p;
     if (!on || pass == P_FWD_HESS || !ctx->fused_inject || p.l != 0 || p.fdorder > 8) return false;
-    if (ctx->sel_fused > 0 || ctx->sel_staged > 0 || ctx->sel_persist > 0) return false;     /* another variant is chosen */
+    if (ctx->sel_fused > 0 || ctx->sel_staged > 0 || (ctx->sel_persist > 0 && !tuned)) return false;   /* another variant is chosen */
     pb->fdorder = p.fdorder; pb->p2 = dh_pow2(p.dh) ? 1 : 0; pb->nx = p.nx; pb->ny = p.ny; pb->fw = p.fw; pb->nb = nb;
     pb->mode = pass == P_ADJ ? TB_ADJ : (pass == P_FWD_STORE || pass == P_RECOMP) ? TB_STORE : TB_FWD;
     pb->max_entries = pass == P_ADJ ? ctx->geo_max_ntr : ctx->geo_max_src;
@@ -1666,7 +1669,7 @@ static bool tblock_cfg(dsh_ctx *ctx, Pass pass, int nb, TbProblem *pb, TbCfg *cf
        4: 1.9 and 4.0; 500 x 200: 2.5 and 4.4; 700 x 280: 3.6 and 4.7; FDORDER 8, k 2:
        3.5 and 4.0, 4.4 and 4.7; 3 shots of 500 x 200 5.3 and 5.1; with one step 1000
        x 300 7.1 and 4.9, 700 x 280, FDORDER 8: 7.2 and 5.5) */
-    const bool asked = ctx->sel_tblock > 0 || env;
+    const bool asked = sel > 0 || env;
     if (!asked && (long long)p.nx * p.ny * nb > 1 << 18) return false;
     pb->min_k = asked ? 1 : 2;
     return tb_config(*pb, cfg);
@@ -2246,6 +2249,7 @@ static void select_variant(dsh_ctx *ctx, int v)
     ctx->sel_persist = v < 0 ? -1 : VARIANT_SEL[v][2];
     ctx->sel_cluster = v < 0 ? -1 : VARIANT_SEL[v][3];
     ctx->sel_tblock = v < 0 ? -1 : VARIANT_SEL[v][4];
+    ctx->sel_tuned = 0;
 }
 
 extern "C" int dsh_set_step_variant(dsh_ctx *ctx, int variant)
@@ -2378,9 +2382,11 @@ extern "C" int dsh_get_field(dsh_ctx *ctx, int shot, int which, float *out)
 
 /* Times plain forward steps of each step-kernel variant the context can run
  * on these shots — kernel pair (v_step), pair with v_step_st, fused step,
- * persistent launch, cluster-resident launch, temporally blocked launches —
- * and keeps the fastest for the context's later calls (the fused choice also
- * serves the gradient passes, the last three only plain forward modelling).
+ * persistent launch, cluster-resident launch, temporally blocked pass — and
+ * keeps the fastest for the context's later calls.  The first three also
+ * serve the other passes; a choice of one of the last three is about plain
+ * forward modelling, and the other passes then run as without a choice
+ * (tblock_cfg: with the blocked pass within its limits, else the pair).
  * ms_per_step[DSH_STEP_VARIANTS] (optional): mean device ms per step of each
  * variant, 0 where it does not apply. */
 extern "C" int dsh_autotune(dsh_ctx *ctx, const dsh_shot *shots, int nshots, int nsteps, float *ms_per_step,
@@ -2423,6 +2429,7 @@ extern "C" int dsh_autotune(dsh_ctx *ctx, const dsh_shot *shots, int nshots, int
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     select_variant(ctx, best);
+    ctx->sel_tuned = 1;
     drop_graphs(ctx);
     if (ms_per_step) for (int v = 0; v < DSH_STEP_VARIANTS; v++) ms_per_step[v] = ms[v];
     if (choice) *choice = best;

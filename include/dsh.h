@@ -192,16 +192,19 @@ int dsh_profile_step(dsh_ctx *ctx, int pass, int nsteps, float *out_ms3);
  * halo of k*(FDORDER-1) points in registers and shared memory and exchanges
  * its halo with the neighbouring tiles every k steps (k up to 8/4/3/2 for
  * FDORDER 2/4/6/8; NX and NY >= 2 FW, at most 1024 source points, 8 sources
- * per point and 2048 receivers per shot).  Without a choice, variant 5 serves
- * the passes it can up to 262144 points over the shots of a launch where k
- * >= 2, and 0 the others. */
+ * per point and 2048 receivers per shot; in the adjoint pass, whose sources
+ * the receivers are, 1024 receivers and 8 at one point).  Without a choice,
+ * variant 5 serves the passes it can up to 262144 points over the shots of a
+ * launch where k >= 2, and 0 the others. */
 #define DSH_STEP_VARIANTS 6
 
 /* Step-kernel autotuner: times nsteps plain forward steps of every variant
  * this context can run on these shots, keeps the fastest for the context's
  * later calls and reports ms_per_step[DSH_STEP_VARIANTS] (0 where a variant
- * does not apply) and *choice.  Results do not depend on the choice (all
- * variants are bit-identical). */
+ * does not apply) and *choice.  A choice of 3, 4 or 5 is about plain forward
+ * passes: the others then run as without a choice (5 within the limits above,
+ * else 0).  Results do not depend on the choice (all variants are
+ * bit-identical). */
 int dsh_autotune(dsh_ctx *ctx, const dsh_shot *shots, int nshots, int nsteps, float *ms_per_step, int *choice);
 
 /* The same for the fused step kernel (one launch per time step; used when
