@@ -35,9 +35,9 @@ __host__ __device__ constexpr bool multi_supported(int fdo, int l)
 }
 
 /* Batches of up to MULTI_PARAM_MODELS models pass every model's StepArgs in
- * the kernel's parameter space (840 B each, within the 32 KB parameter
- * limit): a block reads its model's fields there (constant cache) and starts
- * its loads at once, instead of first copying the 840 B into shared memory
+ * the kernel's parameter space (904 B each; the limit of 32764 B leaves 909
+ * for 36 models): a block reads its model's fields there (constant cache) and
+ * starts its loads at once, instead of first copying them into shared memory
  * behind a block barrier. */
 constexpr int MULTI_PARAM_MODELS = 36;
 struct MultiParams {

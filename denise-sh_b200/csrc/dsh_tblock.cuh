@@ -50,7 +50,8 @@
 
 namespace dsh {
 
-/* block sizes of the builds: 64, 88 and 128 registers per thread */
+/* block sizes of the builds: 64, 80 (704 threads are 22 warps, six on one scheduler) and up to 128 registers per
+ * thread; the first two spill (FDORDER 4: 100-140 and 44-60 bytes stored) */
 constexpr int TB_MAX_THREADS = 1024, TB_MID_THREADS = 704, TB_FEW_THREADS = 512;
 constexpr int TB_MAX_ENT = 1024; /* sources of a slot (receivers in the adjoint) */
 constexpr int TB_MAX_MEM = 8;    /* sources at one point */
