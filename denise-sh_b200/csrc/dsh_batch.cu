@@ -38,6 +38,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <list>
 #include <map>
 #include <memory>
 #include <numeric>
@@ -514,6 +515,9 @@ static int batch_forward(dsh_batch *b, const dsh_shot *shots, const int *nshots,
     }
     for (int k = 0; k < b->n; k++)
         if (nshots[k] > 0 && (rc = zero_slots(b->ctx[k], nshots[k], false)) != DSH_OK) return rc;
+    std::list<CallUse> use;
+    for (dsh_ctx *c : b->ctx) use.emplace_back(c);
+    use_step_kernels(b->ctx[0]);
     b->launches = 0;
     b->points = 0;
     BK(cudaEventRecord(b->ev[0], b->st));

@@ -1370,6 +1370,49 @@ static void v_shape(const dsh_ctx *ctx, const VPick &v, int nb, dim3 *grid, dim3
 /* graph key code of the velocity kernel in use */
 static long long v_code(const dsh_ctx *ctx) { return pick_v(ctx, ctx->p.fdorder, 0, dh_pow2(ctx->p.dh)).code; }
 
+/* What the calls of this process that are in flight on a device run there: SMs
+ * that blocked passes fill (a block keeps its SM for the whole pass), and the
+ * calls that run step kernels.  Blocked passes that do not fit beside each other
+ * take turns, and one among other calls' launches holds both up, where the step
+ * kernels of several contexts overlap.  So without a choice a pass is blocked
+ * where the others in flight are too and all fit.  us per step of all, a thread
+ * per context, FDORDER 4: 8 of 500 x 200 20.0 with blocked passes in turn, 12.9
+ * with one blocked among pairs, 7.7 by this rule (pair 7.4); 4 of 160 x 80 with 8
+ * shots 11.4, 9.2, 7.7 (7.6); two of 160 x 80 with one shot 2.1 (4.3). */
+constexpr int MAX_DEV = 64;
+static struct {
+    std::atomic<int> sms, other;
+} device_use[MAX_DEV];
+
+namespace dsh::eng {
+CallUse::~CallUse()
+{
+    device_use[ctx->dev % MAX_DEV].sms -= ctx->use_sms;
+    device_use[ctx->dev % MAX_DEV].other -= ctx->use_other;
+    ctx->use_sms = ctx->use_other = 0;
+}
+void use_step_kernels(dsh_ctx *ctx)
+{
+    if (!ctx->use_other) device_use[ctx->dev % MAX_DEV].other++;
+    ctx->use_other = 1;
+}
+}  // namespace dsh::eng
+
+/* room for a blocked pass of so many tiles beside the other calls in flight; it then counts until the call ends */
+static bool tb_room(dsh_ctx *ctx, int tiles, bool asked)
+{
+    auto &u = device_use[ctx->dev % MAX_DEV];
+    int nsm = 0;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->dev) != cudaSuccess) return false;
+    const int more = std::max(0, tiles - ctx->use_sms), before = u.sms.fetch_add(more);
+    if (!asked && (u.other > ctx->use_other || before + more > nsm)) {
+        u.sms -= more;
+        return false;
+    }
+    ctx->use_sms += more;
+    return true;
+}
+
 /* The fused step (one kernel per time step, dsh_fused.cuh) serves every pass
  * but the Hessian one when FDORDER <= 8 and injection/sampling are fused;
  * DSH_FUSED=0 selects the velocity + stress kernel pair instead. */
@@ -1777,7 +1820,9 @@ static int run_steps(dsh_ctx *ctx, Pass pass, int nb, int n0, int count)
     if (cluster_cfg(ctx, pass, nb, &ccfg)) return run_cluster(ctx, pass, nb, n0, count, ccfg);
     TbCfg tcfg;
     TbProblem tpb;
-    if (tblock_cfg(ctx, pass, nb, &tpb, &tcfg) && tblock_buffers(ctx, nb, tcfg)) return run_tblock(ctx, pass, nb, n0, count, tpb, tcfg);
+    if (tblock_cfg(ctx, pass, nb, &tpb, &tcfg) && tb_room(ctx, tcfg.tiles, tpb.min_k == 1) && tblock_buffers(ctx, nb, tcfg))
+        return run_tblock(ctx, pass, nb, n0, count, tpb, tcfg);
+    use_step_kernels(ctx);
     if (const int grid = persistent_grid(ctx, pass, nb)) return run_persistent(ctx, pass, nb, n0, count, grid);
     const int rc_side = nb > 1 ? side_stream(&ctx->st2, &ctx->ev_fork, &ctx->ev_join, ctx) : DSH_OK;
     if (rc_side != DSH_OK) return rc_side;
@@ -1989,6 +2034,7 @@ static int forward_impl(dsh_ctx *ctx, const dsh_shot *shots, int nshots, float *
 {
     if (!ctx || !shots || nshots < 0) return DSH_ERR_PARAM;
     if (!ctx->model_set) return DSH_ERR_STATE;
+    CallUse use(ctx);
     CK(cudaSetDevice(ctx->dev));
     CK(cudaEventRecord(ctx->ev[0], ctx->st));
     ctx->launches = 0;
@@ -2032,6 +2078,7 @@ static int gradient_impl(dsh_ctx *ctx, const dsh_shot *shots, int nshots, const 
 {
     if (!ctx || !shots || nshots < 1 || (!obs_host && !obs_dev)) return DSH_ERR_PARAM;
     if (!ctx->model_set) return DSH_ERR_STATE;
+    CallUse use(ctx);
     CK(cudaSetDevice(ctx->dev));
     int rc = ensure_storage(ctx);
     if (rc != DSH_OK) return rc;
@@ -2306,6 +2353,7 @@ extern "C" int dsh_hessian_diag(dsh_ctx *ctx, const dsh_shot *shots, int nshots,
 {
     if (!ctx || !shots || nshots < 1) return DSH_ERR_PARAM;
     if (!ctx->model_set) return DSH_ERR_STATE;
+    CallUse use(ctx);
     CK(cudaSetDevice(ctx->dev));
     const dsh_params &p = ctx->p;
     const long long n = (long long)p.nx * p.ny;
@@ -2398,6 +2446,7 @@ extern "C" int dsh_autotune(dsh_ctx *ctx, const dsh_shot *shots, int nshots, int
 {
     if (!ctx || !shots || nshots < 1 || nsteps < 1) return DSH_ERR_PARAM;
     if (!ctx->model_set) return DSH_ERR_STATE;
+    CallUse use(ctx);
     CK(cudaSetDevice(ctx->dev));
     const int nb = std::min(ctx->S, nshots);
     int rc = upload_batch(ctx, shots, nb, nullptr, nullptr, 0);

@@ -5,6 +5,7 @@
 #include "dsh_dispatch.h"
 #include "dsh_setup.h"
 
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <map>
@@ -93,6 +94,7 @@ struct dsh_ctx {
     long long flags_cap = 0;
     float *d_tb = nullptr;                /* exchange buffers of the temporally blocked pass */
     long long tb_cap = 0;
+    int use_sms = 0, use_other = 0;       /* the current call's part of what runs on the device (CallUse) */
     double *d_part = nullptr, *d_l2 = nullptr;
     unsigned *d_wemax = nullptr;
     std::vector<int> ntr_b;
@@ -151,6 +153,14 @@ int upload_batch(dsh_ctx *ctx, const dsh_shot *shots, int nb, const float *obs_h
 StepArgs step_args(dsh_ctx *ctx, Pass pass);
 InjectArgs inject_args(dsh_ctx *ctx, Pass pass);
 int zero_slots(dsh_ctx *ctx, int nb, bool accumulators);
+/* a call that advances wavefields, until its end: what run_steps counted for it on its device is given back */
+struct CallUse {
+    dsh_ctx *ctx;
+    explicit CallUse(dsh_ctx *c) : ctx(c) {}
+    CallUse(const CallUse &) = delete;
+    ~CallUse();
+};
+void use_step_kernels(dsh_ctx *ctx);       /* the call in progress runs step kernels */
 int forward_steps(dsh_ctx *ctx, int nb);   /* every step of a plain forward pass of slots [0, nb) */
 int copy_seis_out(dsh_ctx *ctx, int nb, float *host_out, float *dev_out);
 int check_status(dsh_ctx *ctx);

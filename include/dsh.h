@@ -195,7 +195,8 @@ int dsh_profile_step(dsh_ctx *ctx, int pass, int nsteps, float *out_ms3);
  * per point and 2048 receivers per shot; in the adjoint pass, whose sources
  * the receivers are, 1024 receivers and 8 at one point).  Without a choice,
  * variant 5 serves the passes it can up to 262144 points over the shots of a
- * launch where k >= 2, and 0 the others. */
+ * launch where k >= 2, as long as other contexts' calls in flight on the device
+ * run blocked passes that fit beside it or none, and 0 the others. */
 #define DSH_STEP_VARIANTS 6
 
 /* Step-kernel autotuner: times nsteps plain forward steps of every variant
