@@ -117,15 +117,15 @@ class Ctx:
         _ck(nnlib().dsh_nn_gemm(M, N, K, _p(A), lda, _p(B), ldb, _p(c32), _p(c16), ldc, _p(bias), int(relu),
                                 splits, _p(part), int(accumulate), _p(self.err), self.st), "dsh_nn_gemm")
 
-    @staticmethod
-    def conv3x3_ok(x, C, N, out):
-        """Whether dsh_nn_conv3x3 takes the call: whole K blocks of 32 channels, 16-byte rows of the output, aligned
-        bases.  Other channel counts and offset tensors go through columns and the GEMM."""
-        return C % 32 == 0 and N % 8 == 0 and x.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
-
     def conv3x3(self, x, B, H, W, C, w, ldw, N, c32=None, c16=None, bias=None, relu=False):
-        _ck(nnlib().dsh_nn_conv3x3(_p(x), B, H, W, C, _p(w), ldw, N, _p(c32), _p(c16), _p(bias), int(relu), _p(self.err),
-                                   self.st), "dsh_nn_conv3x3")
+        """False, and nothing done, where dsh_nn_conv3x3 does not apply: K blocks of 32 channels, output rows and tensors
+        on 16-byte boundaries."""
+        px, p32, p16 = _p(x), _p(c32), _p(c16)
+        if C % 32 or N % 8 or (px | (p32 or 0) | (p16 or 0)) & 15:
+            return False
+        _ck(nnlib().dsh_nn_conv3x3(px, B, H, W, C, _p(w), ldw, N, p32, p16, _p(bias), int(relu), _p(self.err), self.st),
+            "dsh_nn_conv3x3")
+        return True
 
     def check(self):
         self.torch.cuda.synchronize()
@@ -163,8 +163,7 @@ class Conv3x3:
         """x bf16 [P][cin] -> y bf16 [P][cout] (ReLU applied)."""
         ctx = self.ctx
         P = B * H * W
-        if ctx.conv3x3_ok(x, self.cin, self.cout, y):
-            ctx.conv3x3(x, B, H, W, self.cin, self.wb, self.ldk, self.cout, c16=y, bias=self.b, relu=True)
+        if ctx.conv3x3(x, B, H, W, self.cin, self.wb, self.ldk, self.cout, c16=y, bias=self.b, relu=True):
             return
         col = ctx.scratch("col", P * self.ldk, ctx.torch.bfloat16)
         _ck(nnlib().dsh_nn_im2col(_p(x), B, H, W, self.cin, _p(col), self.ldk, ctx.st), "im2col")
@@ -187,9 +186,7 @@ class Conv3x3:
         _ck(nnlib().dsh_nn_transpose(_p(dz), P, self.cout, _p(dzT), ldp, ctx.st), "transpose")
         splits = max(1, min(64, P // 8192))
         ctx.gemm(self.K, self.cout, P, colT, ldp, dzT, ldp, c32=self.gwt, splits=splits, accumulate=True)
-        if dx is not None and ctx.conv3x3_ok(dz, self.cout, self.cin, dx):
-            ctx.conv3x3(dz, B, H, W, self.cout, self.wf, self.ldf, self.cin, c32=dx)
-        elif dx is not None:
+        if dx is not None and not ctx.conv3x3(dz, B, H, W, self.cout, self.wf, self.ldf, self.cin, c32=dx):
             col = ctx.scratch("col", P * self.ldf, torch.bfloat16)
             _ck(nnlib().dsh_nn_im2col(_p(dz), B, H, W, self.cout, _p(col), self.ldf, ctx.st), "im2col")
             ctx.gemm(P, self.cin, 9 * self.cout, col, self.ldf, self.wf, self.ldf, c32=dx)
