@@ -1,7 +1,8 @@
-"""Epilogues of the tensor-core GEMM and of the implicit convolution where some lanes of a warp have nothing to store: rows
-past M, pixels outside the map (a warp holds 2 rows x 16 columns), with several 16-column tensor-memory loads per warp,
-against 64-bit products of the same bf16 operands.  Tolerance: K products added in float, each addition off by at most
-2^-23 of the running sum, which never exceeds the sum of the magnitudes; as much again for the bias and the output."""
+"""U-Net kernels at ragged sizes and other channel counts.  Epilogues of the tensor-core GEMM and of the implicit
+convolution where some lanes of a warp have nothing to store: rows past M, pixels outside the map (a warp holds 2 rows x 16
+columns), with several 16-column tensor-memory loads per warp, against 64-bit products of the same bf16 operands; layers
+and heads that the wide kernels cannot take.  Tolerance: K products added in float, each addition off by at most 2^-23 of
+the running sum, which never exceeds the sum of the magnitudes; as much again for the bias and the output."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -100,3 +101,29 @@ def test_conv_layer_of_any_channel_counts(cin, cout, off):
     dzf = flat(dz, cout)
     _check(layer.gwt.view(K, cout), col.t() @ dzf, col.abs().t() @ dzf.abs(), P)
     _check(layer.gb, dz32.view(P, cout).sum(0), dz32.view(P, cout).abs().sum(0), P)
+
+
+@pytest.mark.parametrize("P,C,off", [(1, 8, 0), (297, 32, 0), (1001, 36, 0), (640, 5, 0), (300, 16, 1), (2000, 248, 0)])
+def test_head_of_any_channel_count(P, C, off):
+    """The 1x1 head and its gradients: 8 channels a load (a multiple of 8), 4 (of 4), else one."""
+    import torch
+
+    from dsh import nn as dnn
+
+    L = dnn.nnlib()
+    g = torch.Generator(device="cuda").manual_seed(P + C)
+    x = torch.empty(P * C + off, dtype=torch.bfloat16, device="cuda")[off:]
+    x.copy_(torch.randn(P * C, device="cuda", generator=g))
+    w, b, dout = (torch.randn(n, device="cuda", generator=g) for n in (C, 1, P))
+    out = torch.full((P + 3,), 7.0, device="cuda")
+    dx = torch.full((P * C + off + 3,), 7.0, device="cuda")[off:]
+    gw, gb, part = torch.zeros(C, device="cuda"), torch.zeros(1, device="cuda"), torch.empty(dnn.RED_BLOCKS * (C + 1), device="cuda")
+    assert L.dsh_nn_head_fwd(x.data_ptr(), P, C, w.data_ptr(), b.data_ptr(), out.data_ptr(), None) == 0
+    assert L.dsh_nn_head_bwd(dout.data_ptr(), x.data_ptr(), P, C, w.data_ptr(), dx.data_ptr(), gw.data_ptr(), gb.data_ptr(),
+                             part.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    xd, wd, dd = x.double().view(P, C), w.double(), dout.double()
+    _check(out[:P], xd @ wd + b.double(), xd.abs() @ wd.abs() + b.double().abs(), C)
+    assert torch.equal(dx[:P * C].view(P, C), dout[:, None] * w) and bool((dx[P * C:] == 7).all()) and bool((out[P:] == 7).all())
+    _check(gw, dd @ xd, dd.abs() @ xd.abs(), P + dnn.RED_BLOCKS)
+    _check(gb[0], dd.sum(), dd.abs().sum(), P + dnn.RED_BLOCKS)
